@@ -728,8 +728,8 @@ def run_accuracy(args, rank, world, local):
     """The plain3d field in zfp's fixed-accuracy mode: variable-length blocks,
     compressed on the device with their start bits and decompressed from
     them (each call ends when its result is complete).  Also times the
-    serial block walk that decoding needs without start bits, on a 64^3
-    field."""
+    block index that decoding needs without start bits, and the serial block
+    walk it stands in for, on a field of a few blocks."""
     import torch
 
     import cuzfp_gb300 as gz
@@ -767,11 +767,11 @@ def run_accuracy(args, rank, world, local):
     enc_ms = sum(ev[3 * i].elapsed_time(ev[3 * i + 1]) for i in range(args.steps)) / args.steps
     dec_ms = sum(ev[3 * i + 1].elapsed_time(ev[3 * i + 2]) for i in range(args.steps)) / args.steps
     ms_per_step = max_over_ranks(enc_ms + dec_ms, world, dev)
-    # the serial walk, on a small field (15^3 = 3,375 blocks: too few for
-    # the parallel index, which starts at 4,096), and the parallel index of
-    # the whole stream, checked against the compressor's start bits
+    # the serial walk, on a small field (3^3 = 27 blocks: too few for the
+    # parallel index, which starts at 33), and the parallel index of the
+    # whole stream, checked against the compressor's start bits
     small = synth.sinusoids_device((60, 60, 60), 16, 32, seed=rank, dtype=torch.float64,
-                                   device=dev)
+                                   device=dev)[:12, :12, :12].contiguous()
     sw = gz.compress_mode(small, mode, cuda_stream=stream)
     gz.index_blocks(sw, small.shape, torch.float64, mode, cuda_stream=stream)
     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -779,7 +779,7 @@ def run_accuracy(args, rank, world, local):
     gz.index_blocks(sw, small.shape, torch.float64, mode, cuda_stream=stream)
     b.record(stream)
     b.synchronize()
-    walk_us = a.elapsed_time(b) * 1e3 / (15 ** 3)
+    walk_us = a.elapsed_time(b) * 1e3 / 27
     idx = gz.index_blocks(words, SHAPE, torch.float64, mode, cuda_stream=stream)
     torch.cuda.synchronize()
     t0 = time.perf_counter()

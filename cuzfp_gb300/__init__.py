@@ -759,10 +759,10 @@ def decompress_mode(words, shape, dtype, mode: Mode, offsets=None, out=None,
 
 
 def index_blocks(words, shape, dtype, mode: Mode, cuda_stream: Any = None):
-    """Every block's start bit in a stream written under `mode`: walkers over
-    segments of the stream whose block chains are joined where they merge
-    (one GPU thread walks short streams, and any stream whose chains do not
-    merge)."""
+    """Every block's start bit in a stream written under `mode`: the bits that
+    look like a block's header parsed in parallel, and the chain of blocks
+    followed through the lengths found (one GPU thread walks streams of a few
+    blocks)."""
     t = _type_of(dtype)
     nx, ny, nz = _dims_of(shape)
     nb = _nblocks(shape)

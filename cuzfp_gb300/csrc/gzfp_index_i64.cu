@@ -1,0 +1,11 @@
+// Parallel block index of general-mode streams of int64_t fields.
+#include "gzfp_index.cuh"
+
+namespace gzfp {
+
+template cudaError_t launch_index_fill<int64_t>(int, const IndexJob&, const IndexLists&,
+                                            const IndexState*, bool, int, cudaStream_t);
+template cudaError_t launch_index_sample<int64_t>(int, const IndexJob&, IndexState*, uint64_t, int,
+                                              cudaStream_t);
+
+}  // namespace gzfp

@@ -6,7 +6,7 @@
 #include <stdint.h>
 
 #include "gzfp_array.cuh"
-#include "gzfp_index_host.h"
+#include "gzfp_index_chain.cuh"
 
 namespace gzfp {
 
@@ -69,29 +69,30 @@ uint32_t block_bound_host(int dims, int P, int ebits, const General& mode);
 // offsets[b] = first + b * maxbits: the start bits of a fixed-rate stream
 cudaError_t launch_fixed_offsets(unsigned long long* offsets, uint64_t n, uint64_t first,
                                  uint32_t maxbits, cudaStream_t s);
-// Parallel index of a general-mode stream (gzfp_modes.cuh): walkers over
-// segments of the stream, their extensions up to the chain they merge with,
-// and the assembly of the true chain's pieces into the block offsets.
-struct IndexJob {
-  const uint64_t* in;
-  uint64_t nwords;
-  General mode;
-  uint64_t first;                // bit of block 0
-  uint64_t seg_bits;             // segment length
-  uint32_t nseg, cap;            // segments, positions a segment's list holds
-  uint32_t ext_cap;              // steps an extension may take
-  unsigned long long* lists;     // nseg * cap block starts, in stream order
-  unsigned long long* counts;    // per segment: entries in its list (cap + 1: overflow)
-  unsigned long long* exits;     // per segment: the walker's first start past its end
-  unsigned long long* info;      // per segment: extension steps, merge segment, merge
-                                 // index, status (0 merged, 1 stream end, 2 failed)
+// Parallel index of a general-mode stream (gzfp_index_chain.cuh): the sample
+// of its exponents, and per batch of segments the table (from headers in
+// the sampled range, or by walks) and the true chain's block starts.
+struct IndexLists {
+  uint32_t* first;   // window bits the link kernels start from
+  uint32_t* count;   // of them
+  uint32_t* next;    // taken so far
+};
+struct IndexLinks {
+  uint32_t n1, n2;               // groups of segments, top groups
+  uint32_t* exits;               // nseg * (win + 1) (index_exit)
+  IndexHop *hops1, *hops2;       // n1, n2 times (win + 1)
+  uint32_t *entry0, *entry1, *entry2;  // nseg, n1, n2: the true chain's entries
+  unsigned long long *base0, *base1, *base2;  // blocks before them
 };
 template <typename T>
-cudaError_t launch_index_walk(int dims, const IndexJob& j, bool extend, cudaStream_t s);
+cudaError_t launch_index_sample(int dims, const IndexJob& j, IndexState* st, uint64_t avg,
+                                int sms, cudaStream_t s);
 template <typename T>
-cudaError_t launch_index_assemble(int dims, const IndexJob& j, const IndexPiece* pieces,
-                                  uint32_t npieces, unsigned long long* offsets, uint64_t nblocks,
-                                  unsigned long long* end, cudaStream_t s);
+cudaError_t launch_index_fill(int dims, const IndexJob& j, const IndexLists& l,
+                              const IndexState* st, bool heads, int sms, cudaStream_t s);
+cudaError_t launch_index_link(const IndexJob& j, const IndexLists& lists, const IndexLinks& l,
+                              int sms, IndexState* st, unsigned long long* offsets,
+                              cudaStream_t s);
 
 cudaError_t launch_place_blocks(const uint64_t* scratch, uint32_t slot_words,
                                 const uint32_t* lengths, const unsigned long long* offsets,

@@ -8,7 +8,6 @@
 
 #include <algorithm>
 #include <mutex>
-#include <vector>
 
 #include "gzfp.h"
 #include "gzfp_host.h"
@@ -28,8 +27,7 @@ struct ModeSpace {
   void* sums = nullptr;     size_t sums_cap = 0;      // scan partials + total; walk end
   void* field = nullptr;    size_t field_cap = 0;     // staged host field
   void* stream = nullptr;   size_t stream_cap = 0;    // staged host stream
-  void* index = nullptr;    size_t index_cap = 0;     // parallel index: lists and per-segment state
-  void* pieces = nullptr;   size_t pieces_cap = 0;    // parallel index: the true chain's pieces
+  void* index = nullptr;    size_t index_cap = 0;     // parallel index: table, lists and links
 };
 ModeSpace g_mode[kMaxDevices];
 
@@ -121,89 +119,153 @@ cudaError_t index_launch(int type, int dims, const uint64_t* in, uint64_t nwords
   }
 }
 
-// The block starts of a device stream by the parallel index
-// (gzfp_modes.cuh): walkers over segments of the stream, joined where their
-// chains merge.  Returns false, with nothing written that counts, when a
-// list overflows or a chain does not merge; the caller then walks serially.
-bool parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* words, uint64_t nwords,
-                    uint64_t nblocks, const gzfp::General& mode, uint64_t first,
-                    uint64_t& end_bit, cudaStream_t s, cudaError_t& err) {
-  err = cudaSuccess;
-  const uint64_t total = nwords * 64;
-  if (nblocks < 4096 || first >= total) return false;  // short streams: the serial walk
-  gzfp::IndexJob j{};
+// Bits of a stream that one batch of the index covers at most: its table
+// takes two bytes per bit.
+constexpr uint64_t kIndexBatchBits = 1ull << 28;
+
+// How often the parallel index widens its range of exponents before it
+// leaves the headers for walks.
+constexpr int kIndexTries = 6;
+
+// The block starts of a device stream in parallel (gzfp_index_chain.cuh)
+// into ms.offsets.  `heads`: from the headers whose exponent field is in the
+// range of st (sampled when it is empty); else by walks.  st: done, or
+// broken (heads only: a block's exponent is out of range), or neither (the
+// stream ends before its blocks).
+cudaError_t parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* words,
+                           uint64_t nwords, uint64_t nblocks, const gzfp::General& mode,
+                           uint64_t first, bool heads, uint32_t bound, gzfp::IndexState& st,
+                           cudaStream_t s) {
+  using namespace gzfp;
+  cudaError_t e;
+  int dev = 0, sms = 0;
+  if ((e = cudaGetDevice(&dev)) ||
+      (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
+    return e;
+  const uint64_t total = nwords * 64, span = total > first ? total - first : 0;
+  st.pos = first;
+  st.count = st.end = st.head = 0;
+  st.done = st.broken = 0;
+  if (!span) return cudaSuccess;  // no stream: nothing done
+  const uint64_t avg = span / nblocks + 1;
+  IndexJob j{};
   j.in = words;
   j.nwords = nwords;
   j.mode = mode;
-  j.first = first;
-  j.nseg = (uint32_t)std::min<uint64_t>(4096, nblocks / 1024);
-  j.seg_bits = (total - first + j.nseg - 1) / j.nseg;
-  j.cap = (uint32_t)(4 * ((nblocks + j.nseg - 1) / j.nseg) + 256);
-  j.ext_cap = 16384;
-  const size_t nseg = j.nseg;
-  const size_t bytes = (nseg * j.cap + 7 * nseg) * 8;
-  if ((err = reserve(ms.index, ms.index_cap, bytes))) return false;
-  j.lists = (unsigned long long*)ms.index;
-  j.counts = j.lists + nseg * j.cap;
-  j.exits = j.counts + nseg;
-  j.info = j.exits + nseg;
-  auto walk = [&](bool extend) {
-    switch (type) {
-      case GZFP_TYPE_FLOAT: return gzfp::launch_index_walk<float>(dims, j, extend, s);
-      case GZFP_TYPE_DOUBLE: return gzfp::launch_index_walk<double>(dims, j, extend, s);
-      case GZFP_TYPE_INT32: return gzfp::launch_index_walk<int32_t>(dims, j, extend, s);
-      default: return gzfp::launch_index_walk<int64_t>(dims, j, extend, s);
-    }
+  j.lo = first;
+  j.nblocks = nblocks;
+  j.zeros = type != GZFP_TYPE_INT32 && type != GZFP_TYPE_INT64 && mode.minbits <= 1;
+  j.win = bound;
+  // Segments of about 24 blocks: the link kernels follow a segment's blocks,
+  // and the segments of a group, one dependent load after another.
+  j.seg_bits = 1024;
+  while (j.seg_bits < 32768 && (j.seg_bits <= bound || j.seg_bits < 16 * avg)) j.seg_bits *= 2;
+  const uint64_t nseg_all = (span + j.seg_bits - 1) / j.seg_bits;
+  const uint32_t per = (uint32_t)std::min<uint64_t>(nseg_all, kIndexBatchBits / j.seg_bits);
+  while ((uint64_t)j.fan * j.fan * j.fan < per) j.fan++;
+  const uint32_t n1 = (per + j.fan - 1) / j.fan, n2 = (n1 + j.fan - 1) / j.fan;
+  // carve the workspace
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t a = at;
+    at += (bytes + 255) / 256 * 256;
+    return a;
   };
-  std::vector<unsigned long long> state(6 * nseg);  // counts, info (exits are not needed)
-  if ((err = walk(false)) || (err = walk(true)) ||
-      (err = cudaMemcpyAsync(state.data(), j.counts, nseg * 8, cudaMemcpyDeviceToHost, s)) ||
-      (err = cudaMemcpyAsync(state.data() + 2 * nseg, j.info, 4 * nseg * 8,
-                             cudaMemcpyDeviceToHost, s)) ||
-      (err = cudaStreamSynchronize(s)))
-    return false;
-  const unsigned long long* counts = state.data();
-  const unsigned long long* info = state.data() + 2 * nseg;
-  // follow the true chain from segment 0 (whose walker starts at block 0)
-  std::vector<gzfp::IndexPiece> pieces;
-  if (!gzfp::index_pieces(nseg, j.cap, counts, info, nblocks, pieces)) return false;
-  if ((err = reserve(ms.pieces, ms.pieces_cap, pieces.size() * sizeof(gzfp::IndexPiece))) ||
-      (err = reserve(ms.offsets, ms.offsets_cap, (size_t)nblocks * 8)) ||
-      (err = reserve(ms.sums, ms.sums_cap, 64)) ||
-      (err = cudaMemcpyAsync(ms.pieces, pieces.data(), pieces.size() * sizeof(gzfp::IndexPiece),
-                             cudaMemcpyHostToDevice, s)))
-    return false;
-  const gzfp::IndexPiece* dp = (const gzfp::IndexPiece*)ms.pieces;
-  unsigned long long* off = (unsigned long long*)ms.offsets;
-  unsigned long long* endp = (unsigned long long*)ms.sums;
-  const uint32_t np = (uint32_t)pieces.size();
-  switch (type) {
-    case GZFP_TYPE_FLOAT: err = gzfp::launch_index_assemble<float>(dims, j, dp, np, off, nblocks, endp, s); break;
-    case GZFP_TYPE_DOUBLE: err = gzfp::launch_index_assemble<double>(dims, j, dp, np, off, nblocks, endp, s); break;
-    case GZFP_TYPE_INT32: err = gzfp::launch_index_assemble<int32_t>(dims, j, dp, np, off, nblocks, endp, s); break;
-    default: err = gzfp::launch_index_assemble<int64_t>(dims, j, dp, np, off, nblocks, endp, s); break;
+  const size_t maps = (size_t)j.win + 1;
+  const size_t a_state = take(sizeof(IndexState)), a_count = take(2 * sizeof(uint32_t)),
+               a_table = take((size_t)per * j.seg_bits * 2), a_first = take(per * (maps + 1) * 4),
+               a_exits = take(per * maps * 4), a_hops1 = take(n1 * maps * sizeof(IndexHop)),
+               a_hops2 = take(n2 * maps * sizeof(IndexHop)),
+               a_entry = take(((size_t)per + n1 + n2) * 4),
+               a_base = take(((size_t)per + n1 + n2) * 8);
+  if ((e = reserve(ms.index, ms.index_cap, at)) ||
+      (e = reserve(ms.offsets, ms.offsets_cap, (size_t)nblocks * 8)))
+    return e;
+  char* base = (char*)ms.index;
+  j.table = (uint16_t*)(base + a_table);
+  uint32_t* counters = (uint32_t*)(base + a_count);
+  const IndexLists lists{(uint32_t*)(base + a_first), counters, counters + 1};
+  IndexLinks l{};
+  l.exits = (uint32_t*)(base + a_exits);
+  l.hops1 = (IndexHop*)(base + a_hops1);
+  l.hops2 = (IndexHop*)(base + a_hops2);
+  l.entry0 = (uint32_t*)(base + a_entry);
+  l.entry1 = l.entry0 + per;
+  l.entry2 = l.entry1 + n1;
+  l.base0 = (unsigned long long*)(base + a_base);
+  l.base1 = l.base0 + per;
+  l.base2 = l.base1 + n1;
+  IndexState* dst = (IndexState*)(base + a_state);
+  if ((e = cudaMemcpyAsync(dst, &st, sizeof st, cudaMemcpyHostToDevice, s))) return e;
+  if (heads && st.field_lo > st.field_hi)
+    e = type == GZFP_TYPE_FLOAT ? launch_index_sample<float>(dims, j, dst, avg, sms, s)
+                                : launch_index_sample<double>(dims, j, dst, avg, sms, s);
+  if (e) return e;
+  for (uint64_t s0 = 0; s0 < nseg_all; s0 += per) {
+    j.lo = first + s0 * j.seg_bits;
+    j.nseg = (uint32_t)std::min<uint64_t>(per, nseg_all - s0);
+    l.n1 = (j.nseg + j.fan - 1) / j.fan;
+    l.n2 = (l.n1 + j.fan - 1) / j.fan;
+    switch (type) {
+      case GZFP_TYPE_FLOAT: e = launch_index_fill<float>(dims, j, lists, dst, heads, sms, s); break;
+      case GZFP_TYPE_DOUBLE: e = launch_index_fill<double>(dims, j, lists, dst, heads, sms, s); break;
+      case GZFP_TYPE_INT32: e = launch_index_fill<int32_t>(dims, j, lists, dst, heads, sms, s); break;
+      default: e = launch_index_fill<int64_t>(dims, j, lists, dst, heads, sms, s); break;
+    }
+    if (e || (e = launch_index_link(j, lists, l, sms, dst, (unsigned long long*)ms.offsets, s)))
+      return e;
   }
-  unsigned long long end = 0;
-  if (err || (err = cudaMemcpyAsync(&end, endp, 8, cudaMemcpyDeviceToHost, s)) ||
-      (err = cudaStreamSynchronize(s)))  // also keeps `pieces` alive for its copy
-    return false;
-  end_bit = end;
-  return true;
+  if ((e = cudaMemcpyAsync(&st, dst, sizeof st, cudaMemcpyDeviceToHost, s))) return e;
+  return cudaStreamSynchronize(s);
 }
 
-// Walk the blocks of a device stream into ms.offsets; *end_bit = the bit
-// after the last block: the parallel index, or one thread walking every
-// block when that cannot join its pieces.  Synchronises `s`.
+// Streams of up to this many blocks are walked by one thread (about 5 us a
+// 4^3 block), less than the parallel index's launches and latency.
+constexpr uint64_t kSerialIndexBlocks = 32;
+
+// The blocks of a device stream into ms.offsets; *end_bit = the bit after
+// the last block (past the stream when it ends before its blocks).
+// Synchronises `s`.
 int walk_blocks(ModeSpace& ms, int type, int dims, const uint64_t* words, uint64_t nwords,
                 const gzfp::Geom& g, const gzfp::General& mode, uint64_t first, uint64_t& end_bit,
                 cudaStream_t s) {
   cudaError_t e;
-  if (parallel_index(ms, type, dims, words, nwords, g.nblocks, mode, first, end_bit, s, e))
-    return GZFP_OK;
-  if (e) return cuda_fail(e, "parallel block index");
   if ((e = reserve(ms.offsets, ms.offsets_cap, (size_t)g.nblocks * 8)) ||
       (e = reserve(ms.sums, ms.sums_cap, 64)))
     return cuda_fail(e, "cudaMalloc(block offsets)");
+  gzfp::General open = mode;  // the most bits a block's code takes
+  open.minbits = 0;
+  const uint32_t code = gzfp::block_bound_host(dims, (int)precision_bits(type), ebits_of(type), open);
+  if (mode.minbits >= code) {  // every block is padded to minbits
+    if ((e = gzfp::launch_fixed_offsets((unsigned long long*)ms.offsets, g.nblocks, first,
+                                        mode.minbits, s)) ||
+        (e = cudaStreamSynchronize(s)))
+      return cuda_fail(e, "block offsets");
+    end_bit = first + g.nblocks * mode.minbits;
+    return GZFP_OK;
+  }
+  if (g.nblocks > kSerialIndexBlocks) {
+    // no headers in integer streams; where zero blocks are padded (minbits
+    // > 1, which no mode sets) a header need not start with a 1
+    bool heads = type != GZFP_TYPE_INT32 && type != GZFP_TYPE_INT64 && mode.minbits <= 1;
+    gzfp::IndexState st{};
+    st.field_lo = ~0u;  // none seen
+    for (int t = 0;; t++) {
+      if ((e = parallel_index(ms, type, dims, words, nwords, g.nblocks, mode, first, heads, code,
+                              st, s)))
+        return cuda_fail(e, "parallel block index");
+      if (!heads || !st.broken) break;
+      const unsigned f = (unsigned)(st.head >> 1) & ((1u << ebits_of(type)) - 1);
+      const bool none = st.field_lo > st.field_hi;
+      st.field_lo = none ? f : std::min(st.field_lo, f);
+      st.field_hi = none ? f : std::max(st.field_hi, f);
+      const unsigned most = type == GZFP_TYPE_DOUBLE ? gzfp::index_most<double>()
+                                                     : gzfp::index_most<float>();
+      heads = t < kIndexTries && st.field_hi - st.field_lo + 8 < most;
+    }
+    end_bit = st.done ? st.end : nwords * 64 + 1;
+    return GZFP_OK;
+  }
   if ((e = index_launch(type, dims, words, nwords, g.nblocks, mode, first,
                         (unsigned long long*)ms.offsets, (unsigned long long*)ms.sums, s)))
     return cuda_fail(e, "block walk launch");

@@ -1,8 +1,8 @@
-// gzfp_index_host.h -- the host step of the parallel index of a
-// general-mode stream (gzfp_modes.cuh, gzfp_modes_api.cu): follow the true
-// chain of block starts from segment 0 through the walkers' merges and cut
-// it into pieces for the assembly kernel.  Plain C++, no CUDA: the CPU tests
-// build it on its own.
+// gzfp_index_host.h -- joining walkers over segments of a general-mode
+// stream on the host: follow the true chain of block starts from segment 0
+// through the walkers' merges and cut it into pieces.  A model of the
+// problem that index_model.cpp checks; the library's index joins its
+// segments on the device (gzfp_index_chain.cuh).
 #pragma once
 
 #include <stdint.h>
