@@ -59,10 +59,11 @@ bool make_geom(unsigned nx, unsigned ny, unsigned nz, gzfp::Geom& g, int& dims) 
 }
 
 // Rows of full blocks move as one vector when every row start is aligned:
-// 16 bytes for 4-byte values, 32 for 8-byte values.
-uint32_t rows_vectorizable(const void* p, unsigned nx, int type) {
+// 16 bytes for 4-byte values, 32 for 8-byte values.  (A 1D field is one row,
+// whatever its length.)
+uint32_t rows_vectorizable(const void* p, unsigned nx, int type, int dims) {
   const uintptr_t a = 4 * scalar_size(type);
-  return (nx % 4 == 0 && (uintptr_t)p % a == 0) ? 1u : 0u;
+  return ((dims == 1 || nx % 4 == 0) && (uintptr_t)p % a == 0) ? 1u : 0u;
 }
 
 bool is_device_pointer(const void* p) {
@@ -268,14 +269,10 @@ int staged(bool decode, int type, int dims, const gzfp::Geom& g, unsigned maxbit
     void* df = dev_field ? (void*)hf : sl.field;
     uint64_t* dw = dev_words ? hw : (uint64_t*)sl.stream;
     gzfp::Geom gs = b.g;
-    gs.vec = rows_vectorizable(df, p.nx, type);
+    gs.vec = rows_vectorizable(df, p.nx, type, dims);
     if (!decode) {
       if (!dev_field && (e = cudaMemcpyAsync(df, hf, fbytes, cudaMemcpyHostToDevice, cs))) {
         st = cuda_fail(e, "cudaMemcpyAsync(field H2D)");
-        break;
-      }
-      if (maxbits % 64 && (e = cudaMemsetAsync(dw, 0, (size_t)(nw * 8), cs))) {
-        st = cuda_fail(e, "cudaMemsetAsync(stream)");  // blocks share edge words
         break;
       }
       if ((e = encode_launch(type, dims, df, gs, maxbits, dw, nw, cs))) {
@@ -334,7 +331,7 @@ int gzfp_compress_bits(int type, unsigned nx, unsigned ny, unsigned nz, unsigned
     const void* hd = dev_data ? data : direct_host_alias(data);
     void* hs = dev_stream ? stream : direct_host_alias(stream);
     if (hd && hs && maxbits % 64 == 0) {
-      g.vec = rows_vectorizable(hd, nx, type);
+      g.vec = rows_vectorizable(hd, nx, type, dims);
       if ((e = encode_launch(type, dims, hd, g, maxbits, (uint64_t*)hs, nwords, s)))
         return cuda_fail(e, "encode kernel launch");
       if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "encode kernel");
@@ -343,11 +340,7 @@ int gzfp_compress_bits(int type, unsigned nx, unsigned ny, unsigned nz, unsigned
     return staged(false, type, dims, g, maxbits, (void*)data, dev_data, (uint64_t*)stream,
                   dev_stream, s);
   }
-  if (maxbits % 64 != 0) {
-    // blocks share boundary words, which the kernel ORs into a zeroed stream
-    if ((e = cudaMemsetAsync(stream, 0, bytes, s))) return cuda_fail(e, "cudaMemsetAsync(stream)");
-  }
-  g.vec = rows_vectorizable(data, nx, type);
+  g.vec = rows_vectorizable(data, nx, type, dims);
   if ((e = encode_launch(type, dims, data, g, maxbits, (uint64_t*)stream, nwords, s)))
     return cuda_fail(e, "encode kernel launch");
   return GZFP_OK;
@@ -374,7 +367,7 @@ int gzfp_decompress_bits(int type, unsigned nx, unsigned ny, unsigned nz, unsign
     void* hd = dev_data ? data : direct_host_alias(data);
     const void* hs = dev_stream ? stream : direct_host_alias(stream);
     if (hd && hs) {
-      g.vec = rows_vectorizable(hd, nx, type);
+      g.vec = rows_vectorizable(hd, nx, type, dims);
       if ((e = decode_launch(type, dims, (const uint64_t*)hs, nwords, g, maxbits, hd, s)))
         return cuda_fail(e, "decode kernel launch");
       if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "decode kernel");
@@ -382,7 +375,7 @@ int gzfp_decompress_bits(int type, unsigned nx, unsigned ny, unsigned nz, unsign
     }
     return staged(true, type, dims, g, maxbits, data, dev_data, (uint64_t*)stream, dev_stream, s);
   }
-  g.vec = rows_vectorizable(data, nx, type);
+  g.vec = rows_vectorizable(data, nx, type, dims);
   e = decode_launch(type, dims, (const uint64_t*)stream, nwords, g, maxbits, data, s);
   if (e) return cuda_fail(e, "decode kernel launch");
   return GZFP_OK;
@@ -401,7 +394,7 @@ void set_strides(gzfp::Geom& g, int dims, int type, const void* p, long long sx,
   g.sy = sy ? sy : (long long)g.nx;
   g.sz = sz ? sz : (long long)g.nx * g.ny;
   const long long a = 4 * (long long)scalar_size(type), S = (long long)scalar_size(type);
-  g.vec = (g.sx == 1 && g.nx % 4 == 0 && (uintptr_t)p % a == 0 && (dims < 2 || (g.sy * S) % a == 0) &&
+  g.vec = (g.sx == 1 && (dims == 1 || g.nx % 4 == 0) && (uintptr_t)p % a == 0 && (dims < 2 || (g.sy * S) % a == 0) &&
            (dims < 3 || (g.sz * S) % a == 0))
               ? 1u
               : 0u;
@@ -435,9 +428,9 @@ int strided_call(bool decode, int type, unsigned nx, unsigned ny, unsigned nz, l
   if (!field || !words) return fail(GZFP_ERR_ARG, "null pointer");
   g.base = base;
   const uint64_t nwords = (base + g.nblocks * maxbits + 63) / 64;
-  // blocks share boundary words (with each other or with the header): the
-  // encoder ORs those into a zeroed stream
-  const bool shared_words = maxbits % 64 || base % 64;
+  // behind a header blocks share boundary words with it or each other: the
+  // encoder ORs those into a zeroed stream (without one its launch sees to it)
+  const bool shared_words = base != 0 && (maxbits % 64 || base % 64);
   const size_t need = (size_t)(nwords * 8);
   if (words_bytes < need)
     return fail(decode ? GZFP_ERR_ARG : GZFP_ERR_CAPACITY,

@@ -67,8 +67,14 @@ GZ_HD Geom make_geom_blocks(uint32_t nx, uint32_t ny, uint32_t nz) {
   return g;
 }
 
+template <int D = 3>
 GZ_HD void block_coords(const Geom& g, uint64_t b, uint32_t& ix, uint32_t& iy, uint32_t& iz) {
   const uint32_t b32 = (uint32_t)b;
+  if (D == 1) {
+    ix = b32;
+    iy = iz = 0;
+    return;
+  }
   const uint32_t r = fast_div(b32, g.dbx);
   ix = b32 - r * g.bx;
   iz = fast_div(r, g.dby);
@@ -255,6 +261,17 @@ struct BitWriter {
     }
     if (n) put(0, n);
   }
+  // the first n bits of a string, zeros past its end
+  template <int N>
+  GZ_HD void put_string(const BitString<N>& c, uint32_t n) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const uint32_t l = umin(n, 64u);
+      if (l) put(c.w[i] & lowmask64(l), l);
+      n -= l;
+    }
+    zeros(n);
+  }
   // the block ends mid-word: hand over the partial last word
   GZ_HD void finish() {
     if (fill) emit();
@@ -302,26 +319,26 @@ struct BitReader {
 
 // ------------------------------------------------------- per-block drivers
 
-template <int D, typename T, bool ALIGNED = false, class Words, class PS>
+template <int D, typename T, bool ALIGNED = false, int NW = code4_words<T>(), class Words, class PS>
 GZ_HD void encode_one(const T* in, const Geom& g, uint64_t b, uint32_t maxbits, Words words,
                       PS& ps) {
   typedef typename FT<T>::UInt UInt;
   constexpr int BS = 1 << (2 * D);
   uint32_t ix, iy, iz;
-  block_coords(g, b, ix, iy, iz);
+  block_coords<D>(g, b, ix, iy, iz);
   UInt raw[BS];
   gather<D, T>(in, g, ix, iy, iz, raw);
   BitWriter<Words, ALIGNED> w(words, g.base + b * (uint64_t)maxbits, maxbits);
-  encode_block<D, T>(raw, maxbits, w, ps);
+  encode_block<D, T, NW>(raw, maxbits, w, ps);
   w.finish();
 }
 
-template <int D, typename T, class Words, class PS>
+template <int D, typename T, int NW = code4_words<T>(), class Words, class PS>
 GZ_HD void decode_one(T* out, const Geom& g, uint64_t b, uint32_t maxbits, Words words, PS& ps) {
   typedef typename FT<T>::UInt UInt;
   constexpr int BS = 1 << (2 * D);
   uint32_t ix, iy, iz;
-  block_coords(g, b, ix, iy, iz);
+  block_coords<D>(g, b, ix, iy, iz);
   BitReader<Words> r(words, g.base + b * (uint64_t)maxbits);
   if constexpr (D == 3 && !FT<T>::INT && sizeof(T) == 8) {
     // 4^3 double blocks hand over their values one z slice at a time, so
@@ -348,7 +365,7 @@ GZ_HD void decode_one(T* out, const Geom& g, uint64_t b, uint32_t maxbits, Words
     return;
   }
   UInt raw[BS];
-  decode_block<D, T>(r, maxbits, raw, ps);
+  decode_block<D, T, NW>(r, maxbits, raw, ps);
   scatter<D, T>(out, g, ix, iy, iz, raw);
 }
 

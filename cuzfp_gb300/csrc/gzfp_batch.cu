@@ -92,7 +92,7 @@ int layout(const gzfp_batch_item* items, int count, bool decode, uint64_t chunk_
         BatchDesc& d = descs[slot++];
         d.g = make_geom_blocks(it.nx, it.ny ? it.ny : 1, it.nz ? it.nz : 1);
         d.g.vec =
-            (it.nx % 4 == 0 && (uintptr_t)it.field % batch_row_align(it.type) == 0) ? 1u : 0u;
+            ((it.nx % 4 == 0 || !it.ny) && (uintptr_t)it.field % batch_row_align(it.type) == 0) ? 1u : 0u;
         d.nwords = (d.g.nblocks * it.maxbits + 63) / 64;
         d.maxbits = it.maxbits;
         d.kind = kBatchKind[k];

@@ -793,7 +793,7 @@ GZ_HD int uncode_flat64(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, Sto
 // (plane k first) spread to every other bit.  Runs at frontier 0 (all-zero
 // planes, one 0 bit each) and 1 are coded and decoded whole; the other
 // planes go one at a time through the small-block coder.  (Used for 2D
-// blocks; 4-value blocks use the plane tables below.)
+// blocks; 4-value blocks have their own coder below.)
 
 // bit i of x (below 2^32) to bit 2i
 GZ_HD uint64_t spread2(uint64_t x) {
@@ -923,22 +923,32 @@ GZ_HD int uncode_runs01(UInt& u0, int k, int k_low, uint32_t& n, uint32_t& bits,
 // (Z/src/template/encode.c:122-151): n verbatim bits, then the group tests,
 // at most 7 bits in all.  Decoding a plane (decode_ints, Z/src/template/
 // decode.c:73-105) reads at most 7 bits and depends only on n, those bits
-// and how many of them the budget still allows.  So both directions are
-// table lookups with no data-dependent branch: the encoder codes two planes
-// per lookup, the decoder one.  A budget that ends inside a plane cuts the
+// and how many of them the budget still allows.  So one plane is a table
+// lookup.  But most planes need none:
+//  * at frontier 3 and 4 a plane's code is its 4 bits, whatever they are (a
+//    fourth coefficient is announced by the test bit and its own one is
+//    implied), so from there on the code is the block's planes, 4 bits each;
+//  * a plane that brings no new coefficient is its n bits and a 0 test, so a
+//    run of such planes at frontier n < 3 is the string of planes with 3 - n
+//    bits left out of every 4.
+// And the frontier only grows, at the planes where a later coefficient has
+// its first one.  A block is therefore at most three runs, a looked-up plane
+// after each, and the rest verbatim: straight-line code, whose steps the
+// lanes of a warp take together.  A budget that ends inside a plane cuts the
 // encoder's output there, as the bit-serial coder stops there; for the
-// decoder the budget is part of the index, and zfp's rule that a run cut
-// off by the budget still deposits a one is in the table.
+// decoder the budget is part of the table's index, and zfp's rule that a run
+// cut off by the budget still deposits a one is in the table.
+// (Two planes per lookup through all planes instead: 1D f32, 2^26 - 3 values
+// at rate 12, took 360 us to encode and 428 us to decode.)
 
 struct Plane4Tables {
-  // planes k and k - 1: index n * 256 + x_k + 16 * x_{k-1}; entry = both
-  // codes (14 bits, plane k's first) | plane k's code length << 14 | both
-  // lengths << 17 | frontier after plane k << 21 | after both << 24
-  uint32_t enc2[5 * 256];
-  // one plane, with r = min(7, bits left) >= 1: index n * 256 + (r == 7 ?
-  // 128 + the next 7 bits : 2^r + the next r bits); entry = the plane's 4
-  // bits | bits read << 4 | frontier after << 7
-  uint16_t dec[5 * 256];
+  // plane x at frontier n < 3: index n * 16 + x; entry = code | length << 7 |
+  // frontier after << 10
+  uint16_t enc[3 * 16];
+  // one plane at frontier n < 3, with r = min(7, bits left) >= 1: index
+  // n * 256 + (r == 7 ? 128 + the next 7 bits : 2^r + the next r bits);
+  // entry = the plane's 4 bits | bits read << 4 | frontier after << 7
+  uint16_t dec[3 * 256];
 };
 
 struct Code4 {
@@ -986,12 +996,10 @@ GZ_CX Code4 plane4_decode(uint32_t v, uint32_t r, uint32_t n) {
 
 GZ_CX Plane4Tables make_plane4_tables() {
   Plane4Tables t{};
-  for (uint32_t n = 0; n <= 4; n++) {
-    for (uint32_t i = 0; i < 256; i++) {
-      const Code4 a = plane4_code(i & 15u, n);
-      const Code4 c = plane4_code(i >> 4, a.n);
-      t.enc2[n * 256 + i] = (a.code | (c.code << a.len)) | (a.len << 14) |
-                            ((a.len + c.len) << 17) | (a.n << 21) | (c.n << 24);
+  for (uint32_t n = 0; n < 3; n++) {
+    for (uint32_t x = 0; x < 16; x++) {
+      const Code4 a = plane4_code(x, n);
+      t.enc[n * 16 + x] = (uint16_t)(a.code | (a.len << 7) | (a.n << 10));
     }
     for (uint32_t r = 1; r <= 7; r++)
       for (uint32_t v = 0; v < (1u << r); v++) {
@@ -1014,92 +1022,300 @@ inline const Plane4Tables* plane4_tables_host() {
   return &t;
 }
 
-// Planes k, k-1, ... down to k_low of a 4-value block while budget
-// remains, from the tables.  k starts at P - 1.  The 4x4 bit tiles of each
-// 32-bit slice of the coefficients are transposed, so word i holds planes
-// 32G + 4c + i at bits 4c..4c+3; the words are shifted up a tile at a time
-// and two planes make one table index.
-template <typename UInt, class W>
-GZ_HD void code_planes_4(const UInt* u, int k, int k_low, uint32_t& n, uint32_t& bits, W& w,
-                         const Plane4Tables& t) {
-  constexpr int NS = (int)sizeof(UInt) / 4;  // 32-bit slices
-  auto pair = [&](uint32_t xb) {  // planes k, k - 1 (xb = x_k | x_{k-1} << 4)
-    if (k < k_low || !bits) return;
-    const uint32_t e = t.enc2[n * 256 + xb];
-    const bool two = k - 1 >= k_low;
-    const uint32_t len = two ? (e >> 17) & 15u : (e >> 14) & 7u;
-    n = two ? (e >> 24) & 7u : (e >> 21) & 7u;
-    const uint32_t l = len < bits ? len : bits;
-    w.put(e & ((1u << l) - 1), l);
-    bits -= l;
-    k -= 2;
-  };
+// Interleave four words bit by bit: bit 4j + i of the 128-bit result is bit
+// j of v[i].  4x4 tiles transposed in place, then bytes across the words,
+// then nibbles within each.  The steps are their own inverses.
+GZ_HD void swap_bytes4(uint32_t* t) {  // byte b of word a <-> byte a of word b
+  const uint32_t a = perm_bytes(t[0], t[1], 0x5140), b = perm_bytes(t[0], t[1], 0x7362);
+  const uint32_t c = perm_bytes(t[2], t[3], 0x5140), d = perm_bytes(t[2], t[3], 0x7362);
+  t[0] = perm_bytes(a, c, 0x5410);
+  t[1] = perm_bytes(a, c, 0x7632);
+  t[2] = perm_bytes(b, d, 0x5410);
+  t[3] = perm_bytes(b, d, 0x7632);
+}
+GZ_HD uint32_t swap_nibbles(uint32_t x) {  // nibbles 1 <-> 2 of each 16 bits
+  const uint32_t t = ((x >> 4) ^ x) & 0x00f000f0u;
+  return x ^ t ^ (t << 4);
+}
+GZ_HD void interleave4(uint32_t* t) {
+  transpose_tiles<4>(t);
+  swap_bytes4(t);
 #pragma unroll
-  for (int G = NS - 1; G >= 0; G--) {
-    uint32_t tw[4];
+  for (int i = 0; i < 4; i++) t[i] = perm_bytes(swap_nibbles(t[i]), 0, 0x3120);
+}
+GZ_HD void deinterleave4(uint32_t* t) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) tw[i] = (uint32_t)((uint64_t)u[i] >> (32 * G));
-    transpose_tiles<4>(tw);
-#pragma unroll 1
-    for (int c = 7; c >= 0 && k >= k_low && bits; c--) {
-      pair((tw[3] >> 28) | ((tw[2] >> 24) & 0xf0u));
-      pair((tw[1] >> 28) | ((tw[0] >> 24) & 0xf0u));
-#pragma unroll
-      for (int i = 0; i < 4; i++) tw[i] <<= 4;
-    }
-  }
+  for (int i = 0; i < 4; i++) t[i] = swap_nibbles(perm_bytes(t[i], 0, 0x3120));
+  swap_bytes4(t);
+  transpose_tiles<4>(t);
 }
 
-// Decode planes k = P - 1, ... down to k_low of a 4-value block while
-// budget remains, from the tables, into u (zero on entry).  The stream is
-// read through a 64-bit window refilled when fewer than 7 bits are left in
-// it; the planes are shifted into the transposed words of code_planes_4.
-template <typename UInt, class R>
-GZ_HD void uncode_planes_4(UInt* u, int k, int k_low, uint32_t& n, uint32_t& bits, R& r,
-                           const Plane4Tables& t) {
-  constexpr int NS = (int)sizeof(UInt) / 4;
-  uint64_t win = r.peek64();
-  uint32_t avail = 64, taken = 0;  // bits of win not yet used; used since the last skip
-  auto one = [&]() -> uint32_t {   // plane k
-    if (k < k_low || !bits) return 0u;
-    if (avail < 7) {
-      r.skip(taken);
-      taken = 0;
-      win = r.peek64();
-      avail = 64;
-    }
-    const uint32_t v = (uint32_t)win & 127u;
-    const uint32_t idx = bits >= 7 ? 128u + v : (1u << bits) + (v & ((1u << bits) - 1));
-    const uint32_t e = t.dec[n * 256 + idx];
-    const uint32_t used = (e >> 4) & 7u;
-    n = e >> 7;
-    win >>= used;
-    avail -= used;
-    taken += used;
-    bits -= used;
-    k--;
-    return e & 15u;
-  };
+// The same for the low 16 bits of four words: 64 bits.
+GZ_HD uint64_t interleave4x16(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+  constexpr uint32_t m = 0x33333333u, k = 0x55555555u, f = 0x0f0f0f0fu;
+  uint32_t p = perm_bytes(v0, v1, 0x5410), q = perm_bytes(v2, v3, 0x5410);
+  uint32_t a = (p & m) | ((q << 2) & ~m), b = ((p >> 2) & m) | (q & ~m);  // rows 0 1, 2 3
+  p = perm_bytes(a, b, 0x5410);  // rows 0 2
+  q = perm_bytes(a, b, 0x7632);  // rows 1 3
+  a = (p & k) | ((q << 1) & ~k);
+  b = ((p >> 1) & k) | (q & ~k);
+  // row i holds planes 4c + i in its nibbles c
+  p = (a & f) | ((b << 4) & ~f);
+  q = ((a >> 4) & f) | (b & ~f);
+  return (uint64_t)perm_bytes(p, q, 0x6420) | ((uint64_t)perm_bytes(p, q, 0x7531) << 32);
+}
+GZ_HD void deinterleave4x16(uint64_t x, uint32_t* v) {
+  constexpr uint32_t m = 0x33333333u, k = 0x55555555u, f = 0x0f0f0f0fu;
+  uint32_t p = perm_bytes(lo32(x), hi32(x), 0x5140), q = perm_bytes(lo32(x), hi32(x), 0x7362);
+  uint32_t a = (p & f) | ((q << 4) & ~f), b = ((p >> 4) & f) | (q & ~f);
+  p = (a & k) | ((b << 1) & ~k);
+  q = ((a >> 1) & k) | (b & ~k);
+  a = perm_bytes(p, q, 0x5410);
+  b = perm_bytes(p, q, 0x7632);
+  p = (a & m) | ((b << 2) & ~m);
+  q = ((a >> 2) & m) | (b & ~m);
+  v[0] = p & 0xffffu;
+  v[1] = p >> 16;
+  v[2] = q & 0xffffu;
+  v[3] = q >> 16;
+}
+
+// bit i of x (below 2^16) to bit 2i, and back (odd bits ignored)
+GZ_HD uint32_t spread16(uint32_t x) {
+  x = (x | (x << 8)) & 0x00ff00ffu;
+  x = (x | (x << 4)) & 0x0f0f0f0fu;
+  x = (x | (x << 2)) & 0x33333333u;
+  return (x | (x << 1)) & 0x55555555u;
+}
+GZ_HD uint32_t compact16(uint32_t x) {
+  x &= 0x55555555u;
+  x = (x | (x >> 1)) & 0x33333333u;
+  x = (x | (x >> 2)) & 0x0f0f0f0fu;
+  x = (x | (x >> 4)) & 0x00ff00ffu;
+  return (x | (x >> 8)) & 0x0000ffffu;
+}
+// bit i of x (below 2^10) to bit 3i, and back (the others ignored)
+GZ_HD uint32_t spread10(uint32_t x) {
+  x = (x | (x << 16)) & 0x030000ffu;
+  x = (x | (x << 8)) & 0x0300f00fu;
+  x = (x | (x << 4)) & 0x030c30c3u;
+  return (x | (x << 2)) & 0x09249249u;
+}
+GZ_HD uint32_t every3rd(uint32_t x) {
+  x &= 0x09249249u;
+  x = (x | (x >> 2)) & 0x030c30c3u;
+  x = (x | (x >> 4)) & 0x0300f00fu;
+  x = (x | (x >> 8)) & 0x030000ffu;
+  return (x | (x >> 16)) & 0x3ffu;
+}
+
+// x >> s, 0 from the type's width on
+GZ_HD uint32_t shr_(uint32_t x, uint32_t s) {
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_rc(x, 0, s);
+#else
+  return s < 32 ? x >> s : 0;
+#endif
+}
+GZ_HD uint64_t shr_(uint64_t x, uint32_t s) { return shr64(x, s); }
+
+// A short bit string in N 64-bit words (registers).
+template <int N>
+struct BitString {
+  uint64_t w[N];
+  // put len (<= 63) bits of v in front; what passes the last word is lost
+  GZ_HD void push(uint64_t v, uint32_t len) {
 #pragma unroll
-  for (int G = NS - 1; G >= 0; G--) {
-    uint32_t tw[4] = {0, 0, 0, 0};
-    int c = 7;
-#pragma unroll 1
-    for (; c >= 0 && k >= k_low && bits; c--) {
-      const uint32_t x3 = one(), x2 = one(), x1 = one(), x0 = one();
-      tw[3] = (tw[3] << 4) | x3;
-      tw[2] = (tw[2] << 4) | x2;
-      tw[1] = (tw[1] << 4) | x1;
-      tw[0] = (tw[0] << 4) | x0;
-    }
-    const uint32_t sh = 4u * (uint32_t)(c + 1);  // tiles not reached are zero
-#pragma unroll
-    for (int i = 0; i < 4; i++) tw[i] = sh < 32 ? tw[i] << sh : 0u;
-    transpose_tiles<4>(tw);
-#pragma unroll
-    for (int i = 0; i < 4; i++) u[i] |= (UInt)((uint64_t)tw[i] << (32 * G));
+    for (int i = N - 1; i > 0; i--) w[i] = (w[i] << len) | ((w[i - 1] >> 1) >> (63 - len));
+    w[0] = (w[0] << len) | v;
   }
-  r.skip(taken);
+  // drop len (<= 63) bits from the front
+  GZ_HD void drop(uint32_t len) {
+#pragma unroll
+    for (int i = 0; i < N - 1; i++) w[i] = (w[i] >> len) | ((w[i + 1] << 1) << (63 - len));
+    w[N - 1] >>= len;
+  }
+  // clear the bits from `len` on
+  GZ_HD void cut(uint32_t len) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      w[i] &= len > 64u * i ? lowmask64(len - 64u * i) : 0;
+  }
+};
+
+// Words that hold the longest code of a 4-value block: header, planes, tests.
+template <typename T>
+GZ_CX int code4_words() { return sizeof(T) == 4 ? 3 : 5; }
+
+// The code of the first np planes (from the top) of a 4-value block, its
+// first 64 N bits, put together from its end: every piece is pushed in front
+// of what follows it, so no piece has to find its place and a budget cuts
+// nothing until the end.  Returns the length (uncut).
+template <int N, typename UInt>
+GZ_HD uint32_t code_planes_4(const UInt* u, uint32_t np, const Plane4Tables& t,
+                             BitString<N>& code) {
+  UInt v[4];  // plane j at bit j
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = brev_u(u[i]);
+  auto clz = [](UInt x) { return sizeof(UInt) == 8 ? clz64((uint64_t)x) : clz32((uint32_t)x); };
+  auto bit = [&](int i, uint32_t j) { return (uint32_t)shr_(v[i], j) & 1u; };
+  // plane j at frontier n, by table: its entry, of no length past the last
+  auto plane = [&](uint32_t j, uint32_t n) -> uint32_t {
+    const uint32_t x = bit(0, j) + 2 * bit(1, j) + 4 * bit(2, j) + 8 * bit(3, j);
+    return j < np ? t.enc[n * 16 + x] : n << 10;
+  };
+  // forwards: the runs and the planes after them.  j1, j2: the runs' starts
+  const UInt u23 = u[2] | u[3], u123 = u[1] | u23;
+  const uint32_t j0 = umin(clz((UInt)(u[0] | u123)), np);
+  const uint32_t e0 = plane(j0, 0);
+  const uint32_t j1 = j0 + 1;
+  uint32_t n = e0 >> 10, r1 = 0, e1 = n << 10, j2 = j1;
+  if (n == 1) {  // planes of the first coefficient alone: its bit, 0
+    const uint32_t k = umin(clz(u123), np);
+    r1 = k > j1 ? k - j1 : 0;
+    e1 = plane(k, 1);
+    j2 = k + 1;
+    n = e1 >> 10;
+  }
+  uint32_t r2 = 0, e2 = n << 10, j3 = j2;
+  if (n == 2) {  // of the first two: their bits, 0
+    const uint32_t k = umin(clz(u23), np);
+    r2 = k > j2 ? k - j2 : 0;
+    e2 = plane(k, 2);
+    j3 = k + 1;
+  }
+  // backwards: the verbatim planes, then every piece in front
+  uint32_t len = np > j3 ? 4 * (np - j3) : 0;
+  UInt x[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) x[i] = shr_(v[i], j3);
+  if constexpr (N == 1) {
+    code.w[0] = interleave4x16((uint32_t)x[0], (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) code.w[i] = 0;
+#pragma unroll
+    for (int h = 0; 2 * h < N - 1 && h < (int)sizeof(UInt) / 4; h++) {
+      uint32_t q[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) q[i] = (uint32_t)((uint64_t)x[i] >> (32 * h));
+      interleave4(q);
+      code.w[2 * h] = (uint64_t)q[0] | ((uint64_t)q[1] << 32);
+      code.w[2 * h + 1] = (uint64_t)q[2] | ((uint64_t)q[3] << 32);
+    }
+  }
+  if (np < 8 * sizeof(UInt)) code.cut(len);  // planes the block does not code
+  auto push = [&](uint64_t c, uint32_t l) {
+    code.push(c, l);
+    len += l;
+  };
+  push(e2 & 127u, (e2 >> 7) & 7u);
+  for (uint32_t r = r2; r;) {
+    const uint32_t c = (r - 1) % 10 + 1, m = (1u << c) - 1;  // the last 1..10 of them
+    r -= c;
+    push(spread10((uint32_t)shr_(v[0], j2 + r) & m) |
+             (spread10((uint32_t)shr_(v[1], j2 + r) & m) << 1), 3 * c);
+  }
+  push(e1 & 127u, (e1 >> 7) & 7u);
+  for (uint32_t r = r1; r;) {
+    const uint32_t c = (r - 1) % 16 + 1;
+    r -= c;
+    push(spread16((uint32_t)shr_(v[0], j1 + r) & ((1u << c) - 1)), 2 * c);
+  }
+  push(e0 & 127u, (e0 >> 7) & 7u);
+  if (sizeof(UInt) == 8 && j0 > 63) {
+    push(0, 63);
+    push(0, j0 - 63);
+  } else {
+    push(0, j0);
+  }
+  return len;
+}
+
+// Decode the first np planes of a 4-value block from its code (the bits past
+// the budget zero) into u.  v holds the coefficients bit-reversed: plane j at
+// bit j.
+template <int N, typename UInt>
+GZ_HD void uncode_planes_4(UInt* u, uint32_t np, uint32_t& bits, BitString<N>& code,
+                           const Plane4Tables& t) {
+  constexpr uint32_t kShift = 8 * sizeof(UInt) - 1;
+  UInt v[4] = {0, 0, 0, 0};
+  uint32_t j = 0, n = 0;
+  auto take = [&](uint32_t c) {
+    code.drop(c);
+    bits -= c;
+  };
+  auto plane = [&]() {  // plane j, by table
+    if (j >= np || !bits) return;
+    const uint32_t w = lo32(code.w[0]) & 127u;  // 0 past the budget
+    const uint32_t e = t.dec[n * 256 + (bits >= 7 ? 128u : 1u << bits) + w];
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] |= (UInt)((e >> i) & 1u) << j;
+    take((e >> 4) & 7u);
+    n = e >> 7;
+    j++;
+  };
+  // all-zero planes, then the first that is not
+  for (uint32_t c;; ) {
+    const uint32_t w = lo32(code.w[0]);
+    c = umin(w ? ctz32(w) : 32u, umin(np - j, bits));
+    take(c);
+    j += c;
+    if (c < 32 || j >= np || !bits) break;
+  }
+  plane();
+  if (n == 1) {  // planes of the first coefficient alone, up to a 1 test
+    uint32_t c;
+    do {
+      const uint32_t w = lo32(code.w[0]), hit = w & 0xaaaaaaaau;
+      c = umin(hit ? ctz32(hit) >> 1 : 16u, umin(np - j, bits >> 1));
+      v[0] |= (UInt)(compact16(w) & ((1u << c) - 1)) << (j & kShift);
+      j += c;
+      take(2 * c);
+    } while (c == 16 && j < np && bits > 1);
+    plane();
+  }
+  if (n == 2) {  // of the first two
+    uint32_t c;
+    do {
+      const uint32_t w = lo32(code.w[0]), hit = w & 0x24924924u;
+      c = hit ? (ctz32(hit) * 43) >> 7 : 10u;  // a third of it
+      c = umin(c, np - j);
+      c = 3 * c > bits ? bits / 3 : c;
+      const uint32_t m = (1u << c) - 1;
+      v[0] |= (UInt)(every3rd(w) & m) << (j & kShift);
+      v[1] |= (UInt)(every3rd(w >> 1) & m) << (j & kShift);
+      j += c;
+      take(3 * c);
+    } while (c == 10 && j < np && bits > 2);
+    plane();
+  }
+  // verbatim; the last plane may be cut by the budget
+  if (j < np && bits) {
+    const uint32_t left = umin(4 * (np - j), bits);
+    if (np < 8 * sizeof(UInt)) code.cut(left);
+    bits -= left;
+    UInt x[4] = {0, 0, 0, 0};
+    if constexpr (N == 1) {
+      uint32_t q[4];
+      deinterleave4x16(code.w[0], q);
+#pragma unroll
+      for (int i = 0; i < 4; i++) x[i] = q[i];
+    } else {
+#pragma unroll
+      for (int h = 0; 2 * h < N - 1 && h < (int)sizeof(UInt) / 4; h++) {
+        uint32_t q[4] = {lo32(code.w[2 * h]), hi32(code.w[2 * h]), lo32(code.w[2 * h + 1]),
+                         hi32(code.w[2 * h + 1])};
+        deinterleave4(q);
+#pragma unroll
+        for (int i = 0; i < 4; i++) x[i] |= (UInt)((uint64_t)q[i] << (32 * h));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] |= x[i] << j;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = brev_u(v[i]);
 }
 
 // --------------------------------------------------------- float <-> bits
@@ -1394,7 +1610,10 @@ struct General {
 // 4^3 double blocks are coded one 32-bit slice (32 planes) at a time; the
 // bottom slice waits in plane-store slots 32..63 while the top one is coded,
 // so only half of the block's coefficients stay in registers.
-template <int D, typename T, class Mode, class W, class PS>
+//
+// NW: 64-bit words of a 1D block's code that are wanted (all by default; a
+// fixed-rate caller with a smaller budget asks for fewer).
+template <int D, typename T, int NW = code4_words<T>(), class Mode, class W, class PS>
 GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mode, W& w,
                                  PS& ps) {
   typedef FT<T> F;
@@ -1405,7 +1624,7 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
   const uint32_t maxbits = mode.maxbits;
 
   UInt u[BS];
-  uint32_t bits;
+  uint32_t bits, head = 0;
   int kmin;
   if constexpr (F::INT) {
     front_end_int<D, T>(raw, u);
@@ -1438,7 +1657,8 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
       }
     }
     const uint32_t e = (uint32_t)(emax + F::EBIAS);
-    w.put(2 * (uint64_t)e + 1, F::EBITS + 1);
+    if constexpr (D != 1) w.put(2 * (uint64_t)e + 1, F::EBITS + 1);
+    head = 2 * e + 1;
     front_end<D, T>(raw, emax, u);
     bits = maxbits - (F::EBITS + 1);
     kmin = P - prec;
@@ -1462,7 +1682,23 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
     planes_to_store<0>(u, ps);
     code_planes<BS>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
   } else if constexpr (D == 1) {
-    code_planes_4(u, k, kmin, n, bits, w, *ps.t4);
+    BitString<NW> code;
+    uint32_t len = code_planes_4(u, (uint32_t)(P - kmin), *ps.t4, code);
+    if constexpr (!F::INT) {
+      code.push(head, F::EBITS + 1);
+      len += F::EBITS + 1;
+    }
+    (void)bits;
+    if constexpr (!Mode::kGeneral) {
+      w.put_string(code, maxbits);
+      return maxbits;
+    } else {
+      const uint32_t used = umin(len, maxbits);
+      const uint32_t all = used < mode.minbits ? mode.minbits : used;
+      code.cut(used);
+      w.put_string(code, all);
+      return all;
+    }
   } else {
     PL pl;
 #pragma unroll
@@ -1497,9 +1733,9 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
   }
 }
 
-template <int D, typename T, class W, class PS>
+template <int D, typename T, int NW = code4_words<T>(), class W, class PS>
 GZ_HD void encode_block(const typename FT<T>::UInt* raw, uint32_t maxbits, W& w, PS& ps) {
-  encode_block_mode<D, T>(raw, FixedRate{maxbits}, w, ps);
+  encode_block_mode<D, T, NW>(raw, FixedRate{maxbits}, w, ps);
 }
 
 // Decode one block from a reader positioned at its first bit into raw IEEE
@@ -1513,8 +1749,9 @@ struct NoSlice {
 
 // SLICED (4^3 floating-point blocks): the values of z slice z go to
 // slice(z, 16 values) as soon as they are final, and raw is not written.
-template <int D, typename T, bool SLICED = false, class Mode, class R, class PS,
-          class SliceFn = NoSlice>
+// NW as for encode_block_mode.
+template <int D, typename T, bool SLICED = false, int NW = code4_words<T>(), class Mode, class R,
+          class PS, class SliceFn = NoSlice>
 GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* raw, PS& ps,
                                  SliceFn&& slice = SliceFn{}) {
   typedef FT<T> F;
@@ -1577,9 +1814,16 @@ GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* r
       store_to_coeffs<0>(ps, 0, k, top, u);
     }
   } else if constexpr (D == 1) {
+    BitString<NW> code;
+    uint32_t left = bits;
 #pragma unroll
-    for (int i = 0; i < BS; i++) u[i] = 0;
-    uncode_planes_4(u, k, kmin, n, bits, r, *ps.t4);
+    for (int i = 0; i < NW; i++) {
+      const uint32_t c = umin(left, 64u);
+      code.w[i] = c ? r.peek64() & lowmask64(c) : 0;
+      if (i + 1 < NW) r.skip(c);
+      left -= c;
+    }
+    uncode_planes_4(u, (uint32_t)(P - kmin), bits, code, *ps.t4);
   } else {
 #pragma unroll
     for (int i = 0; i < PL::NW; i++) ps.put(i, 0);
@@ -1633,9 +1877,9 @@ GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* r
   return used < mode.min_bits() ? mode.min_bits() : used;
 }
 
-template <int D, typename T, class R, class PS>
+template <int D, typename T, int NW = code4_words<T>(), class R, class PS>
 GZ_HD void decode_block(R& r, uint32_t maxbits, typename FT<T>::UInt* raw, PS& ps) {
-  decode_block_mode<D, T>(r, FixedRate{maxbits}, raw, ps);
+  decode_block_mode<D, T, false, NW>(r, FixedRate{maxbits}, raw, ps);
 }
 
 // The bits a block takes in a general-mode stream, from a reader at its

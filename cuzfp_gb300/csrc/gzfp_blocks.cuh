@@ -92,7 +92,7 @@ cudaError_t launch_encode_blocks_t(const T* tiles, const unsigned long long* ind
                                    uint64_t* out, uint64_t nwords, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
   const dim3 grid((unsigned)((count + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(store_slots<D, T>(), false, 0, table_words<D>());
+  const size_t sm = smem_bytes(store_slots<D, T>(), kStageNone, 0, table_words<D>());
   auto k = encode_blocks_kernel<D, T>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
@@ -107,7 +107,7 @@ cudaError_t launch_decode_blocks_t(const uint64_t* in, uint64_t nwords,
                                    uint64_t count, uint32_t maxbits, T* tiles, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
   const dim3 grid((unsigned)((count + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(decode_slots<D, T>(), false, 0, table_words<D>());
+  const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0, table_words<D>());
   auto k = decode_blocks_kernel<D, T>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;

@@ -29,7 +29,7 @@ int ebits_of(int type);                       // block-header exponent bits (0 f
 size_t scalar_size(int type);
 // geometry of nx x ny x nz (ny = 0: 1D, nz = 0: 2D), under 2^32 blocks
 bool make_geom(unsigned nx, unsigned ny, unsigned nz, gzfp::Geom& g, int& dims);
-uint32_t rows_vectorizable(const void* p, unsigned nx, int type);
+uint32_t rows_vectorizable(const void* p, unsigned nx, int type, int dims);
 bool is_device_pointer(const void* p);
 int check_common(int type, unsigned nx, unsigned ny, unsigned nz, unsigned maxbits,
                  gzfp::Geom& g, int& dims);

@@ -6,10 +6,9 @@
 // Decode: the inverse, reading the slot and storing the valid values.
 //
 // Shared memory per CTA: each thread's plane store (the coder walks planes in
-// a rolled loop), and, when every block fills whole 64-bit words ("staged"
-// mode, maxbits % 64 == 0), a word buffer: the decoder's warp loads its 32
-// consecutive stream slots into it with coalesced loads, and the encoder's
-// warp assembles its slots there and stores them with coalesced stores.
+// a rolled loop), and a word buffer in which the stream's words are staged
+// (kStage*): the decoder loads them with coalesced loads, and the encoder
+// assembles them there and stores them with coalesced stores.
 //
 // Replaces cuZFP's cudaEncode / cudaEncode1 / cudaEncode2 and cudaDecode /
 // cudaDecode1 / cudaDecode2 (src/cuZFP/encode{1,2,3}.cuh, decode{1,2,3}.cuh).
@@ -26,11 +25,30 @@ constexpr int kStride = kThreads + 1;    // staged word buffer row pitch (words)
 constexpr uint32_t kMaxStagedWords = 64; // staged decode up to 4096-bit blocks
 constexpr uint32_t kMaxStagedOut = 16;   // staged encoder output up to 1024-bit blocks
 constexpr uint32_t kPadRows = 2;         // zero rows after each staged slot
+// How a CTA reaches the stream's words.
+// kStageNone: in place; the encoder ORs the words that neighbouring blocks
+// share into a zeroed stream.
+// kStageRows: blocks of whole words, word j of thread t's block at
+// buf[j * kStride + t], so that the lanes of a warp hit different banks.
+// kStageRun: the words of the CTA's 128 blocks in stream order.  These begin
+// and end on word boundaries whatever the block's size is, so words are
+// shared within the CTA only: no zeroing of the stream, no global atomics.
+// 4-value blocks take it up to two words (their slots are short, so the
+// lanes' words spread over the banks), others where blocks are not whole words.
+// Against words reached in place, with the same coder (compress / decompress):
+// 1D f32, 2^25 - 3 values, rate 12, 176 -> 121 / 177 -> 130 us; 1D f64, 2^24
+// - 3, rate 12, 150 -> 90 / 137 -> 84; 2D f32 4093 x 4095, rate 11.3, 132 ->
+// 126 / 145 -> 124; 3D f64 256^3, rate 15.3, 139 -> 133 / 126 -> 103; 3D f32
+// 256^3, rate 15.3, 100 -> 92 / 77 -> 69.  (1D f64, rate 48: 154 -> 155 / 148
+// -> 158.)
+constexpr int kStageNone = 0, kStageRows = 1, kStageRun = 2;
+
 // dynamic shared memory of a CTA: the plane store (up to 32 slots of 8
-// bytes per thread) and, when staged, the word buffer
-inline size_t smem_bytes(int slots, bool staged, uint32_t words_per_block, int tables = 0) {
+// bytes per thread), the tables, and the word buffer
+inline size_t smem_bytes(int slots, int stage, uint32_t maxbits, int tables = 0) {
   size_t b = ((size_t)slots * kThreads + (size_t)tables) * 8;
-  if (staged) b += (size_t)(words_per_block + kPadRows) * kStride * 8;
+  if (stage == kStageRows) b += (size_t)((maxbits >> 6) + kPadRows) * kStride * 8;
+  if (stage == kStageRun) b += (size_t)(kThreads / 64 * maxbits + kPadRows) * 8;
   return b;
 }
 
@@ -44,7 +62,7 @@ struct SmemPlanes {
 };
 
 // 4-value blocks code through the plane tables, which each CTA copies into
-// the start of its shared memory (7.5 KB); other blocks use none.
+// the start of its shared memory (1.6 KB); other blocks use none.
 template <int D>
 __host__ __device__ constexpr int table_words() {
   return D == 1 ? (int)(sizeof(Plane4Tables) / 8) : 0;
@@ -92,6 +110,66 @@ struct StagedWords {
   __device__ __forceinline__ uint64_t load(uint64_t i) const {
     uint64_t j = i - w0;
     return j < W ? buf[j * PITCH] : 0;
+  }
+};
+
+// The words of a CTA's blocks in stream order in shared memory, zero at
+// first: a word that neighbouring blocks share is merged with atomics on its
+// halves.
+struct RunWords {
+  uint64_t* buf;
+  uint64_t w0;  // global index of the first word
+};
+template <>
+struct BitWriter<RunWords, false> {
+  uint64_t* buf;
+  uint64_t acc;
+  uint32_t wi, fill, first, last;  // as the general writer's, within the buffer
+  __device__ __forceinline__ BitWriter(RunWords w, uint64_t pos, uint32_t maxbits) : buf(w.buf), acc(0) {
+    const uint32_t p = (uint32_t)(pos - (w.w0 << 6)), end = p + maxbits;
+    wi = p >> 6;
+    fill = p & 63;
+    first = fill ? wi : ~0u;
+    last = end & 63 ? end >> 6 : ~0u;
+  }
+  __device__ __forceinline__ void emit() {
+    if (wi == first || wi == last) {
+      uint32_t* h = reinterpret_cast<uint32_t*>(buf + wi);
+      if (lo32(acc)) atomicOr(h, lo32(acc));
+      if (hi32(acc)) atomicOr(h + 1, hi32(acc));
+    } else {
+      buf[wi] = acc;
+    }
+    wi++;
+  }
+  __device__ __forceinline__ void put(uint64_t v, uint32_t n) {
+    acc |= v << fill;
+    const uint32_t f = fill + n;
+    if (f >= 64) {
+      emit();
+      acc = (v >> 1) >> (63 - fill);
+      fill = f - 64;
+    } else {
+      fill = f;
+    }
+  }
+  // the first n bits of a string, as the whole block (which starts at fill)
+  template <int N>
+  __device__ __forceinline__ void put_string(BitString<N> c, uint32_t n) {
+    c.cut(n);
+    uint64_t low = 0;
+#pragma unroll
+    for (int i = 0; i <= N; i++) {
+      if ((uint32_t)(64 * i) >= fill + n) break;
+      acc = (i < N ? c.w[i] << fill : 0) | ((low >> 1) >> (63 - fill));
+      low = i < N ? c.w[i] : 0;
+      emit();
+    }
+    fill = 0;
+  }
+  __device__ __forceinline__ void zeros(uint32_t) {}  // ends the block; the buffer is zero
+  __device__ __forceinline__ void finish() {
+    if (fill) emit();
   }
 };
 
@@ -146,9 +224,11 @@ __device__ __forceinline__ void warp_copy(uint64_t* buf, uint64_t* gwords, uint3
 
 // Register budget: the 4^3 double kernels keep a whole block (64 x 64 bits)
 // in registers; 168 registers per thread allow 3 CTAs of 128 threads per SM.
+// The 1D kernels need few, and left to itself the compiler takes more (79
+// for the float encoder: 22 warps per SM and 68% of the ALU pipe).
 template <int D, typename T>
 struct MinBlocks {
-  static constexpr int value = (D == 3 && sizeof(T) == 8) ? 3 : 4;
+  static constexpr int value = D == 1 ? (sizeof(T) == 8 ? 10 : 16) : D == 3 && sizeof(T) == 8 ? 3 : 4;
 };
 
 // Plane-store slots per thread, as many as the block codec touches, so that
@@ -165,20 +245,20 @@ __host__ __device__ constexpr int decode_slots() {
   return D == 3 ? 32 : store_slots<D, T>();
 }
 
-// ALIGNED: every block fills whole words (maxbits % 64 == 0, no header
-// offset); its words are then assembled in the staged buffer and the warp
-// stores its 32 consecutive slots with coalesced stores.
-template <int D, typename T, bool ALIGNED = false>
+// NW: words of a 1D block's code (encode_block_mode).
+template <int D, typename T, int STAGE = kStageNone, int NW = code4_words<T>()>
 __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
     encode_kernel(const T* __restrict__ in, Geom g, uint32_t maxbits, uint64_t* __restrict__ out,
                   uint64_t nwords) {
   extern __shared__ uint64_t smem[];
+  uint64_t* buf = smem + table_words<D>() + store_slots<D, T>() * kThreads;
+  if constexpr (STAGE == kStageRun)
+    for (uint32_t i = threadIdx.x; i < kThreads / 64 * maxbits; i += kThreads) buf[i] = 0;
   const Plane4Tables* t4 = stage_tables<D, kThreads>(smem);
   SmemPlanes ps{smem + table_words<D>() + threadIdx.x, t4};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if constexpr (ALIGNED) {
+  if constexpr (STAGE == kStageRows) {
     const uint32_t W = maxbits >> 6;
-    uint64_t* buf = smem + table_words<D>() + store_slots<D, T>() * kThreads;
     if (b < g.nblocks)
       encode_one<D, T, true>(in, g, b, maxbits, StagedWords<kStride>{buf + threadIdx.x, b * W, W}, ps);
     __syncwarp();
@@ -187,6 +267,14 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
       const uint64_t left = g.nblocks - b0;
       warp_copy<true>(buf + (threadIdx.x & ~31u), out + b0 * W, W, left < 32 ? (uint32_t)left : 32);
     }
+  } else if constexpr (STAGE == kStageRun) {
+    const uint64_t w0 = (uint64_t)blockIdx.x * (kThreads / 64) * maxbits;
+    if (D != 1) __syncthreads();  // (the tables' staging ends with one)
+    if (b < g.nblocks) encode_one<D, T, false, NW>(in, g, b, maxbits, RunWords{buf, w0}, ps);
+    __syncthreads();
+    const uint64_t left = nwords - w0;
+    const uint32_t n = left < kThreads / 64 * maxbits ? (uint32_t)left : kThreads / 64 * maxbits;
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads) out[w0 + i] = buf[i];
   } else {
     if (b < g.nblocks)
       encode_one<D, T>(in, g, b, maxbits, DevWords{out, nullptr, nwords}, ps);
@@ -196,17 +284,23 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
 // MINB: resident CTAs per SM the register budget is sized for.  The decoder
 // is latency-bound on its plane chain, so a fourth CTA is worth a tighter
 // register budget whenever shared memory allows one (dec_min_blocks).
-template <int D, typename T, bool STAGED, int MINB>
+template <int D, typename T, int STAGE, int MINB, int NW = code4_words<T>()>
 __global__ void __launch_bounds__(kThreads, MINB)
     decode_kernel(const uint64_t* __restrict__ in, uint64_t nwords, Geom g, uint32_t maxbits,
                   T* __restrict__ out) {
   extern __shared__ uint64_t smem[];
+  uint64_t* buf = smem + table_words<D>() + decode_slots<D, T>() * kThreads;
+  const uint64_t w0 = (uint64_t)blockIdx.x * (kThreads / 64) * maxbits;
+  if constexpr (STAGE == kStageRun) {
+    const uint64_t left = nwords - w0;
+    for (uint32_t i = threadIdx.x; i < kThreads / 64 * maxbits + kPadRows; i += kThreads)
+      buf[i] = i < left ? __ldg(in + w0 + i) : 0;
+  }
   const Plane4Tables* t4 = stage_tables<D, kThreads>(smem);
   SmemPlanes ps{smem + table_words<D>() + threadIdx.x, t4};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (STAGED) {
+  if constexpr (STAGE == kStageRows) {
     const uint32_t W = maxbits >> 6;
-    uint64_t* buf = smem + table_words<D>() + decode_slots<D, T>() * kThreads;
     const uint64_t b0 = b - (threadIdx.x & 31);
     if (b0 < g.nblocks) {
       const uint64_t left = g.nblocks - b0;
@@ -218,29 +312,44 @@ __global__ void __launch_bounds__(kThreads, MINB)
     __syncwarp();
     if (b < g.nblocks)
       decode_one<D, T>(out, g, b, maxbits, StagedWords<kStride>{buf + threadIdx.x, b * W, W}, ps);
+  } else if constexpr (STAGE == kStageRun) {
+    if (D != 1) __syncthreads();
+    if (b < g.nblocks)
+      decode_one<D, T, NW>(out, g, b, maxbits, StagedWords<1>{buf, w0, kThreads / 64 * maxbits}, ps);
   } else {
     if (b < g.nblocks) decode_one<D, T>(out, g, b, maxbits, DevWords{nullptr, in, nwords}, ps);
   }
 }
 
-// kernel launchers shared by the per-type translation units
+// Kernel launchers shared by the per-type translation units.  The encoder
+// stages blocks of up to kMaxStagedOut words when their buffer fits beside
+// the plane store without costing a resident CTA (larger blocks measured
+// faster with direct stores).
 template <int D, typename T>
 cudaError_t launch_encode_t(const T* in, const Geom& g, uint32_t maxbits, uint64_t* out,
                             uint64_t nwords, cudaStream_t s) {
   if (g.nblocks == 0) return cudaSuccess;
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
-  // staged output for blocks of up to kMaxStagedOut words, when they fit
-  // beside the plane store without costing a resident CTA (larger blocks
-  // measured faster with direct stores)
   constexpr int MB = MinBlocks<D, T>::value;
-  const bool aligned =
-      maxbits % 64 == 0 && g.base == 0 && (maxbits >> 6) <= kMaxStagedOut &&
-      (smem_bytes(store_slots<D, T>(), true, maxbits >> 6, table_words<D>()) + 1024) * MB <=
-          227 * 1024;
-  const size_t sm = smem_bytes(store_slots<D, T>(), aligned, maxbits >> 6, table_words<D>());
-  auto k = aligned ? encode_kernel<D, T, true> : encode_kernel<D, T>;
+  int stage = D == 1 || maxbits % 64 ? kStageRun : kStageRows;
+  if (g.base != 0 || maxbits > 64 * kMaxStagedOut ||
+      (smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D>()) + 1024) * MB > 227 * 1024)
+    stage = kStageNone;
+  const size_t sm = smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D>());
+  auto k = stage == kStageRun ? encode_kernel<D, T, kStageRun> : encode_kernel<D, T, kStageNone>;
+  if constexpr (D == 1) {  // no more words of code than the budget
+    if (stage == kStageRun && maxbits <= 128)
+      k = maxbits <= 64 ? encode_kernel<D, T, kStageRun, 1> : encode_kernel<D, T, kStageRun, 2>;
+  } else if (stage == kStageRows) {
+    k = encode_kernel<D, T, kStageRows>;
+  }
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
+  // blocks that share words in place: into a zeroed stream (with a header,
+  // the caller has zeroed it and written the header)
+  if (stage == kStageNone && g.base == 0 && maxbits % 64 &&
+      (e = cudaMemsetAsync(out, 0, (size_t)nwords * 8, s)) != cudaSuccess)
+    return e;
   k<<<grid, kThreads, sm, s>>>(in, g, maxbits, out, nwords);
   return cudaGetLastError();
 }
@@ -254,12 +363,26 @@ cudaError_t launch_decode_t(const uint64_t* in, uint64_t nwords, const Geom& g, 
                             T* out, cudaStream_t s) {
   if (g.nblocks == 0) return cudaSuccess;
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
-  const bool staged = maxbits % 64 == 0 && (maxbits >> 6) <= kMaxStagedWords && g.base == 0;
-  const size_t sm = smem_bytes(decode_slots<D, T>(), staged, maxbits >> 6, table_words<D>());
   constexpr int MB = MinBlocks<D, T>::value;
-  auto k = !staged ? decode_kernel<D, T, false, MB>
-           : (MB < 4 && sm <= kSmemFor4) ? decode_kernel<D, T, true, 4>
-                                         : decode_kernel<D, T, true, MB>;
+  int stage = kStageNone;
+  if (g.base == 0 && maxbits % 64 == 0 && (maxbits >> 6) <= kMaxStagedWords) stage = kStageRows;
+  // a run's buffer must not cost a resident CTA
+  if (g.base == 0 && (maxbits % 64 != 0 || (D == 1 && maxbits <= 128)) &&
+      (smem_bytes(decode_slots<D, T>(), kStageRun, maxbits, table_words<D>()) + 1024) * MB <=
+          227 * 1024)
+    stage = kStageRun;
+  const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D>());
+  auto k = stage == kStageNone   ? decode_kernel<D, T, kStageNone, MB>
+           : stage == kStageRows ? decode_kernel<D, T, kStageRows, MB>
+                                 : decode_kernel<D, T, kStageRun, MB>;
+  if constexpr (MB < 4) {
+    if (sm <= kSmemFor4 && stage != kStageNone)
+      k = stage == kStageRows ? decode_kernel<D, T, kStageRows, 4> : decode_kernel<D, T, kStageRun, 4>;
+  }
+  if constexpr (D == 1) {
+    if (stage == kStageRun && maxbits <= 128)
+      k = maxbits <= 64 ? decode_kernel<D, T, kStageRun, MB, 1> : decode_kernel<D, T, kStageRun, MB, 2>;
+  }
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   k<<<grid, kThreads, sm, s>>>(in, nwords, g, maxbits, out);

@@ -382,7 +382,7 @@ int compress_mode_impl(int type, unsigned nx, unsigned ny, unsigned nz, const gz
     din = ms.field;
   }
   gzfp::Geom gv = g;
-  gv.vec = rows_vectorizable(din, nx, type);
+  gv.vec = rows_vectorizable(din, nx, type, dims);
   if ((e = encode_mode_launch(type, dims, din, gv, gm, (uint64_t*)ms.scratch, slot_words,
                               (uint32_t*)ms.lengths, s)))
     return cuda_fail(e, "encode kernel launch");
@@ -472,7 +472,7 @@ int decompress_mode_impl(int type, unsigned nx, unsigned ny, unsigned nz, const 
     dout = ms.field;
   }
   gzfp::Geom gv = g;
-  gv.vec = rows_vectorizable(dout, nx, type);
+  gv.vec = rows_vectorizable(dout, nx, type, dims);
   st = GZFP_OK;
   if ((e = decode_mode_launch(type, dims, dw, nwords, doff, gv, gm, dout, s)))
     st = cuda_fail(e, "decode kernel launch");
