@@ -48,7 +48,9 @@ inline int batch_kind_index(uint32_t kind) {
 template <int NT>
 struct BatchPlanes {
   uint64_t* p;
-  const Plane4Tables* t4;  // the CTA's plane tables (1D kinds)
+  const Plane4Tables* t4;
+  const GroupTable* gt;
+  __device__ __forceinline__ BatchPlanes(uint64_t* p_, const Tables& t) : p(p_), t4(t.t4), gt(t.gt) {}
   __device__ __forceinline__ uint64_t get(int i) const { return p[i * NT]; }
   __device__ __forceinline__ void put(int i, uint64_t v) { p[i * NT] = v; }
 };
@@ -159,11 +161,12 @@ __global__ void __launch_bounds__(NT, MINB)
     batch_grid_kernel(const BatchDesc* __restrict__ descs,
                       const uint32_t* __restrict__ chunk_item, uint64_t lo, int bpt,
                       uint32_t staged_w) {
-  extern __shared__ uint64_t smem[];
+  extern __shared__ __align__(16) uint64_t smem[];
   __shared__ BatchDesc s_desc;
-  const Plane4Tables* t4 = stage_tables<D, NT>(smem);
-  BatchPlanes<NT> ps{smem + table_words<D>() + threadIdx.x, t4};
-  uint64_t* sbuf = smem + table_words<D>() + BatchSlots<DECODE, D, T>::value * NT;
+  const Tables tables = stage_tables<D, T, DECODE, NT>(smem);
+  tables_ready<D, T, DECODE>();
+  BatchPlanes<NT> ps{smem + table_words<D, T, DECODE>() + threadIdx.x, tables};
+  uint64_t* sbuf = smem + table_words<D, T, DECODE>() + BatchSlots<DECODE, D, T>::value * NT;
   const uint32_t j = blockIdx.x % (uint32_t)bpt;
   const uint64_t chunk = lo + blockIdx.x / (uint32_t)bpt;
   if (threadIdx.x == 0) s_desc = descs[chunk_item[chunk]];
@@ -183,12 +186,13 @@ __global__ void __launch_bounds__(NT, MINB)
     batch_kernel(const BatchDesc* __restrict__ descs, const uint32_t* __restrict__ chunk_item,
                  uint64_t lo, uint64_t hi, unsigned long long* counter, int bpt, int ahead,
                  uint32_t staged_w) {
-  extern __shared__ uint64_t smem[];
+  extern __shared__ __align__(16) uint64_t smem[];
   __shared__ unsigned long long s_claim;
   __shared__ BatchDesc s_desc;  // the claimed chunk's array, read field by field
-  const Plane4Tables* t4 = stage_tables<D, NT>(smem);
-  BatchPlanes<NT> ps{smem + table_words<D>() + threadIdx.x, t4};
-  uint64_t* sbuf = smem + table_words<D>() + BatchSlots<DECODE, D, T>::value * NT;
+  const Tables tables = stage_tables<D, T, DECODE, NT>(smem);
+  tables_ready<D, T, DECODE>();
+  BatchPlanes<NT> ps{smem + table_words<D, T, DECODE>() + threadIdx.x, tables};
+  uint64_t* sbuf = smem + table_words<D, T, DECODE>() + BatchSlots<DECODE, D, T>::value * NT;
   if (threadIdx.x == 0) s_claim = lo + atomicAdd(counter, 1ull);
   __syncthreads();
   for (;;) {
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(NT, MINB)
 // pitch NT + 1)
 template <int NT, bool DECODE, int D, typename T>
 GZ_HD size_t batch_smem_bytes(uint32_t staged_w) {
-  return ((size_t)NT * BatchSlots<DECODE, D, T>::value + (size_t)table_words<D>()) * 8 +
+  return ((size_t)NT * BatchSlots<DECODE, D, T>::value + (size_t)table_words<D, T, DECODE>()) * 8 +
          (staged_w ? (size_t)(staged_w + kPadRows) * (NT + 1) * 8 : 0);
 }
 

@@ -52,35 +52,61 @@ inline size_t smem_bytes(int slots, int stage, uint32_t maxbits, int tables = 0)
   return b;
 }
 
-// per-thread plane store in shared memory, slot i at planes[i * kThreads];
-// t4: the CTA's copy of the 4-value plane tables (1D kernels only)
+// Tables that a coder's CTAs copy into the start of their shared memory: the
+// 4-value plane tables (1D, 1.6 KB) and the group table (4^3 decoders of
+// 64-bit values, 4 KB).
+struct Tables {
+  const Plane4Tables* t4;
+  const GroupTable* gt;
+};
+template <int D, typename T, bool DECODE>
+__host__ __device__ constexpr int table_words() {
+  return D == 1 ? (int)(sizeof(Plane4Tables) / 8)
+         : DECODE && uses_group_table<D, T>() ? (int)(sizeof(GroupTable) / 8)
+                                              : 0;
+}
+
+// Start copying the coder's tables into shared memory (16 bytes aligned),
+// and wait for them: the CTA's own staging goes between the two, so that the
+// copies' latencies overlap.  Every thread of the CTA must call both before
+// any thread returns; tables_ready is a CTA barrier where there are tables
+// (and where ALWAYS is set).
+template <int D, typename T, bool DECODE, int NT>
+__device__ __forceinline__ Tables stage_tables(uint64_t* smem) {
+  constexpr int n = table_words<D, T, DECODE>() / 2;  // 16-byte pieces
+  if constexpr (n == 0) {
+    return Tables{nullptr, nullptr};
+  } else {
+    const char* src = D == 1 ? reinterpret_cast<const char*>(&kPlane4Tables)
+                             : reinterpret_cast<const char*>(&kGroupTable);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+#pragma unroll
+    for (int i = threadIdx.x; i < n; i += NT)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i),
+                   "l"(src + 16 * i) : "memory");
+    return Tables{reinterpret_cast<const Plane4Tables*>(smem),
+                  reinterpret_cast<const GroupTable*>(smem)};
+  }
+}
+template <int D, typename T, bool DECODE, bool ALWAYS = false>
+__device__ __forceinline__ void tables_ready() {
+  if constexpr (table_words<D, T, DECODE>() > 0) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  } else if constexpr (ALWAYS) {
+    __syncthreads();
+  }
+}
+
+// per-thread plane store in shared memory, slot i at planes[i * kThreads]
 struct SmemPlanes {
   uint64_t* p;
   const Plane4Tables* t4;
+  const GroupTable* gt;
+  __device__ __forceinline__ SmemPlanes(uint64_t* p_, const Tables& t) : p(p_), t4(t.t4), gt(t.gt) {}
   __device__ __forceinline__ uint64_t get(int i) const { return p[i * kThreads]; }
   __device__ __forceinline__ void put(int i, uint64_t v) { p[i * kThreads] = v; }
 };
-
-// 4-value blocks code through the plane tables, which each CTA copies into
-// the start of its shared memory (1.6 KB); other blocks use none.
-template <int D>
-__host__ __device__ constexpr int table_words() {
-  return D == 1 ? (int)(sizeof(Plane4Tables) / 8) : 0;
-}
-
-// Copy the plane tables into shared memory and return them (null for
-// D > 1).  Every thread of the CTA must call it before any thread returns.
-template <int D, int NT>
-__device__ __forceinline__ const Plane4Tables* stage_tables(uint64_t* smem) {
-  if constexpr (D != 1) {
-    return nullptr;
-  } else {
-    const uint64_t* src = reinterpret_cast<const uint64_t*>(&kPlane4Tables);
-    for (int i = threadIdx.x; i < table_words<1>(); i += NT) smem[i] = src[i];
-    __syncthreads();
-    return reinterpret_cast<const Plane4Tables*>(smem);
-  }
-}
 
 // Global stream words.  `merge` ORs a word that neighbouring zfp blocks share
 // (only when maxbits is not a multiple of 64; the stream is zeroed first).
@@ -250,12 +276,13 @@ template <int D, typename T, int STAGE = kStageNone, int NW = code4_words<T>()>
 __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
     encode_kernel(const T* __restrict__ in, Geom g, uint32_t maxbits, uint64_t* __restrict__ out,
                   uint64_t nwords) {
-  extern __shared__ uint64_t smem[];
-  uint64_t* buf = smem + table_words<D>() + store_slots<D, T>() * kThreads;
+  extern __shared__ __align__(16) uint64_t smem[];
+  uint64_t* buf = smem + table_words<D, T, false>() + store_slots<D, T>() * kThreads;
+  const Tables tables = stage_tables<D, T, false, kThreads>(smem);
   if constexpr (STAGE == kStageRun)
     for (uint32_t i = threadIdx.x; i < kThreads / 64 * maxbits; i += kThreads) buf[i] = 0;
-  const Plane4Tables* t4 = stage_tables<D, kThreads>(smem);
-  SmemPlanes ps{smem + table_words<D>() + threadIdx.x, t4};
+  tables_ready<D, T, false, STAGE == kStageRun>();
+  SmemPlanes ps{smem + table_words<D, T, false>() + threadIdx.x, tables};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if constexpr (STAGE == kStageRows) {
     const uint32_t W = maxbits >> 6;
@@ -269,7 +296,6 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
     }
   } else if constexpr (STAGE == kStageRun) {
     const uint64_t w0 = (uint64_t)blockIdx.x * (kThreads / 64) * maxbits;
-    if (D != 1) __syncthreads();  // (the tables' staging ends with one)
     if (b < g.nblocks) encode_one<D, T, false, NW>(in, g, b, maxbits, RunWords{buf, w0}, ps);
     __syncthreads();
     const uint64_t left = nwords - w0;
@@ -288,16 +314,16 @@ template <int D, typename T, int STAGE, int MINB, int NW = code4_words<T>()>
 __global__ void __launch_bounds__(kThreads, MINB)
     decode_kernel(const uint64_t* __restrict__ in, uint64_t nwords, Geom g, uint32_t maxbits,
                   T* __restrict__ out) {
-  extern __shared__ uint64_t smem[];
-  uint64_t* buf = smem + table_words<D>() + decode_slots<D, T>() * kThreads;
+  extern __shared__ __align__(16) uint64_t smem[];
+  uint64_t* buf = smem + table_words<D, T, true>() + decode_slots<D, T>() * kThreads;
   const uint64_t w0 = (uint64_t)blockIdx.x * (kThreads / 64) * maxbits;
+  const Tables tables = stage_tables<D, T, true, kThreads>(smem);
   if constexpr (STAGE == kStageRun) {
     const uint64_t left = nwords - w0;
     for (uint32_t i = threadIdx.x; i < kThreads / 64 * maxbits + kPadRows; i += kThreads)
       buf[i] = i < left ? __ldg(in + w0 + i) : 0;
   }
-  const Plane4Tables* t4 = stage_tables<D, kThreads>(smem);
-  SmemPlanes ps{smem + table_words<D>() + threadIdx.x, t4};
+  SmemPlanes ps{smem + table_words<D, T, true>() + threadIdx.x, tables};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if constexpr (STAGE == kStageRows) {
     const uint32_t W = maxbits >> 6;
@@ -310,13 +336,15 @@ __global__ void __launch_bounds__(kThreads, MINB)
 #pragma unroll
     for (uint32_t j = 0; j < kPadRows; j++) buf[(W + j) * kStride + threadIdx.x] = 0;
     __syncwarp();
+    tables_ready<D, T, true>();
     if (b < g.nblocks)
       decode_one<D, T>(out, g, b, maxbits, StagedWords<kStride>{buf + threadIdx.x, b * W, W}, ps);
   } else if constexpr (STAGE == kStageRun) {
-    if (D != 1) __syncthreads();
+    tables_ready<D, T, true, true>();
     if (b < g.nblocks)
       decode_one<D, T, NW>(out, g, b, maxbits, StagedWords<1>{buf, w0, kThreads / 64 * maxbits}, ps);
   } else {
+    tables_ready<D, T, true>();
     if (b < g.nblocks) decode_one<D, T>(out, g, b, maxbits, DevWords{nullptr, in, nwords}, ps);
   }
 }
@@ -333,9 +361,9 @@ cudaError_t launch_encode_t(const T* in, const Geom& g, uint32_t maxbits, uint64
   constexpr int MB = MinBlocks<D, T>::value;
   int stage = D == 1 || maxbits % 64 ? kStageRun : kStageRows;
   if (g.base != 0 || maxbits > 64 * kMaxStagedOut ||
-      (smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D>()) + 1024) * MB > 227 * 1024)
+      (smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D, T, false>()) + 1024) * MB > 227 * 1024)
     stage = kStageNone;
-  const size_t sm = smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D>());
+  const size_t sm = smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D, T, false>());
   auto k = stage == kStageRun ? encode_kernel<D, T, kStageRun> : encode_kernel<D, T, kStageNone>;
   if constexpr (D == 1) {  // no more words of code than the budget
     if (stage == kStageRun && maxbits <= 128)
@@ -368,10 +396,10 @@ cudaError_t launch_decode_t(const uint64_t* in, uint64_t nwords, const Geom& g, 
   if (g.base == 0 && maxbits % 64 == 0 && (maxbits >> 6) <= kMaxStagedWords) stage = kStageRows;
   // a run's buffer must not cost a resident CTA
   if (g.base == 0 && (maxbits % 64 != 0 || (D == 1 && maxbits <= 128)) &&
-      (smem_bytes(decode_slots<D, T>(), kStageRun, maxbits, table_words<D>()) + 1024) * MB <=
+      (smem_bytes(decode_slots<D, T>(), kStageRun, maxbits, table_words<D, T, true>()) + 1024) * MB <=
           227 * 1024)
     stage = kStageRun;
-  const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D>());
+  const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D, T, true>());
   auto k = stage == kStageNone   ? decode_kernel<D, T, kStageNone, MB>
            : stage == kStageRows ? decode_kernel<D, T, kStageRows, MB>
                                  : decode_kernel<D, T, kStageRun, MB>;

@@ -38,9 +38,10 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
                        uint32_t* __restrict__ lengths) {
   typedef typename FT<T>::UInt UInt;
   constexpr int BS = 1 << (2 * D);
-  extern __shared__ uint64_t smem[];
-  const Plane4Tables* t4 = stage_tables<D, kThreads>(smem);
-  SmemPlanes ps{smem + table_words<D>() + threadIdx.x, t4};
+  extern __shared__ __align__(16) uint64_t smem[];
+  const Tables tables = stage_tables<D, T, false, kThreads>(smem);
+  tables_ready<D, T, false>();
+  SmemPlanes ps{smem + table_words<D, T, false>() + threadIdx.x, tables};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if (b >= g.nblocks) return;
   uint32_t ix, iy, iz;
@@ -64,9 +65,10 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
                        T* __restrict__ out) {
   typedef typename FT<T>::UInt UInt;
   constexpr int BS = 1 << (2 * D);
-  extern __shared__ uint64_t smem[];
-  const Plane4Tables* t4 = stage_tables<D, kThreads>(smem);
-  SmemPlanes ps{smem + table_words<D>() + threadIdx.x, t4};
+  extern __shared__ __align__(16) uint64_t smem[];
+  const Tables tables = stage_tables<D, T, true, kThreads>(smem);
+  tables_ready<D, T, true>();
+  SmemPlanes ps{smem + table_words<D, T, true>() + threadIdx.x, tables};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if (b >= g.nblocks) return;
   uint32_t ix, iy, iz;
@@ -102,7 +104,7 @@ cudaError_t launch_encode_mode_t(const T* in, const Geom& g, const General& mode
                                  cudaStream_t s) {
   if (g.nblocks == 0) return cudaSuccess;
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(store_slots<D, T>(), kStageNone, 0, table_words<D>());
+  const size_t sm = smem_bytes(store_slots<D, T>(), kStageNone, 0, table_words<D, T, false>());
   auto k = encode_mode_kernel<D, T>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
@@ -116,7 +118,7 @@ cudaError_t launch_decode_mode_t(const uint64_t* in, uint64_t nwords,
                                  const General& mode, T* out, cudaStream_t s) {
   if (g.nblocks == 0) return cudaSuccess;
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0, table_words<D>());
+  const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0, table_words<D, T, true>());
   auto k = decode_mode_kernel<D, T>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;

@@ -53,10 +53,11 @@ template <bool DECODE, int D, typename T, int MINB, int PATH>
 __global__ void __maxnreg__(queue_maxnreg(MINB))
     serve_request_kernel(const __grid_constant__ BatchDesc d, uint32_t p, uint32_t staged_w,
                          QueueDev q) {
-  extern __shared__ uint64_t smem[];
-  const Plane4Tables* t4 = stage_tables<D, kQThreads>(smem);
-  BatchPlanes<kQThreads> ps{smem + table_words<D>() + threadIdx.x, t4};
-  uint64_t* sbuf = smem + table_words<D>() + BatchSlots<DECODE, D, T>::value * kQThreads;
+  extern __shared__ __align__(16) uint64_t smem[];
+  const Tables tables = stage_tables<D, T, DECODE, kQThreads>(smem);
+  tables_ready<D, T, DECODE>();
+  BatchPlanes<kQThreads> ps{smem + table_words<D, T, DECODE>() + threadIdx.x, tables};
+  uint64_t* sbuf = smem + table_words<D, T, DECODE>() + BatchSlots<DECODE, D, T>::value * kQThreads;
   if (threadIdx.x == 0) atomicMin(&q.t_first[p], queue_clock());
   batch_block<kQThreads, DECODE, D, T, PATH>(d, (uint64_t)blockIdx.x * kQThreads + threadIdx.x,
                                              ps, sbuf, staged_w);
