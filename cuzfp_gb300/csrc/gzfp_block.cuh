@@ -462,6 +462,12 @@ GZ_HD uint64_t rank_spread(uint64_t z) {
   return S;
 }
 
+// A plane's group tests from its rank spread S: 1 | 2 S | 4 (S - top), with
+// disjoint bits; top: 2^(position of the last one after the spread).
+GZ_HD uint64_t group_code(uint64_t S, uint32_t last) {
+  return 6 * S + 1 - (4ull << (last & 63));
+}
+
 // Rank spread of a plane of at most 16 bits: below 2^31.
 GZ_HD uint32_t rank_spread32(uint32_t z) {
   const uint32_t z1 = z & (z - 1);
@@ -492,71 +498,77 @@ GZ_HD int code_planes_small(int k, int k_low, uint32_t& n, uint32_t& bits, W& w,
       encode_plane<BS>(x, n, bits, w);
       continue;
     }
-    const uint32_t xh = full ? 0u : x >> n;
-    const uint32_t hb = bl - 1 - n;
+    const uint32_t xh = any ? x >> n : 0u;
     const uint32_t m = popcount32(xh);
-    const uint32_t S = rank_spread32(xh);
-    const uint64_t grp =
-        any ? (1 | ((uint64_t)S << 1) | ((uint64_t)(S - (1u << ((hb + m - 1) & 31))) << 2)) : 0;
-    const uint32_t hlen = full ? (uint32_t)BS : n;
-    const uint32_t head = full ? x : x & ((1u << n) - 1);
-    const uint32_t glen = full ? 0 : any ? hb + m + 2 : 1;
+    const uint32_t hb = bl - n;             // bits above the frontier
+    const uint64_t grp = any ? group_code(rank_spread32(xh), hb + m - 2) : 0;
+    // the ones above the frontier give way to their group tests
+    uint64_t code = x + ((grp - xh) << n);
+    uint32_t len = n + (any ? hb + m + 1 : full ? 0u : 1u);
     n = any ? bl : n;
-    const uint32_t len = hlen + glen;
-    const uint32_t l = len < bits ? len : bits;
-    w.put(((uint64_t)head | (grp << hlen)) & lowmask64(l), l);
-    bits -= l;
+    if (len > bits) {
+      len = bits;
+      code &= lowmask64(len);
+    }
+    w.put(code, len);
+    bits -= len;
   }
   return k;
 }
 
 // Code planes k, k-1, ... down to k_low while budget remains; plane(k)
-// yields plane k.  Returns the index of the next plane.  A plane's code is
-// written as two pieces -- its n verbatim bits, then its group tests (at
-// most 64 bits) -- so the loop body has no data-dependent branch except the
-// rare general path (a one implied by the last position, or group tests
-// longer than 64 bits), and the 32 threads of a warp (32 blocks) stay
-// converged plane after plane.  A budget that ends inside a plane just
-// truncates its code, as the bit-serial coder does.
-template <int BS, class W, class PlaneFn>
+// yields plane k.  Returns the index of the next plane.  The frontier after a
+// plane is max(n, bit length of the plane), so the chain from one plane to the
+// next is a single max; the rest of a plane's code depends on n but not on the
+// previous plane's code.  A plane without new coefficients is its bits and a 0
+// test; otherwise the ones above the frontier give way to their group tests,
+// in one word with the verbatim bits where both fit (most planes).  A budget
+// that ends inside a plane just truncates its code, as the bit-serial coder
+// does.  CUT: by a branch that few planes take, instead of a mask on each
+// (faster for 32-bit values, 3D f32 320^3 smooth at rate 8 106 -> 104 us, not
+// for doubles, rate 16 200 -> 202).
+// Planes without new coefficients in any lane, the whole of a dense block's
+// last ones, skip the group code: with it computed for every plane 3D i64
+// 320^3 noisy at rate 32 took 316 us, with the branch 244.
+template <int BS, bool CUT = false, class W, class PlaneFn>
 GZ_HD int code_planes(int k, int k_low, uint32_t& n, uint32_t& bits, W& w, PlaneFn&& plane) {
   if constexpr (BS <= 16) return code_planes_small<BS>(k, k_low, n, bits, w, plane);
-  // The frontier after a plane is max(n, bit length of the plane), so the
-  // chain from one plane to the next is a single max; the rest of a plane's
-  // code depends on n but not on the previous plane's code.
   for (; k >= k_low && bits; k--) {
     const uint64_t x = plane(k);
-    const uint32_t bl = 64 - clz64(x);              // bit length of the plane
-    const bool full = n == (uint32_t)BS;            // all significant: plane verbatim
-    const bool any = bl > n;                        // a one above the frontier
-    const uint32_t sh = full ? 0 : n;
-    const uint64_t xh = full ? 0 : x >> sh;         // ones above the frontier
-    const uint32_t hb = bl - 1 - n;                 // top one, relative to the frontier
-    const uint32_t m = (uint32_t)popcount64(xh);
-    if (any && (bl >= (uint32_t)BS || hb + m > 62)) {
-      encode_plane<BS>(x, n, bits, w);
-      continue;
+    const uint32_t bl = 64 - clz64(x);    // bit length of the plane
+    uint64_t code = x;                    // without new ones: verbatim bits, then a 0 test
+    uint32_t len = n + (n == (uint32_t)BS ? 0u : 1u);
+    if (bl > n) {  // ones above the frontier (skipped where no lane has any)
+      const uint64_t xh = x >> n;
+      const uint32_t hb = bl - n, m = (uint32_t)popcount64(xh), g = hb + m + 1;
+      if (bl >= (uint32_t)BS || g > 64) {
+        encode_plane<BS>(x, n, bits, w);
+        continue;
+      }
+      const uint64_t grp = group_code(rank_spread(xh), hb + m - 2);
+      len = n + g;
+      if (len > 64) {  // verbatim bits, then group tests
+        const uint32_t h = umin(n, bits), l = umin(g, bits - h);
+        w.put(x & lowmask64(h), h);
+        w.put(grp & lowmask64(l), l);
+        bits -= h + l;
+        n = bl;
+        continue;
+      }
+      code += (grp - xh) << n;  // the ones give way to their group tests
+      n = bl;
     }
-    const uint64_t S = rank_spread(xh);
-    const uint64_t grp = any ? (1 | (S << 1) | ((S - (1ull << ((hb + m - 1) & 63))) << 2)) : 0;
-    const uint32_t hlen = full ? (uint32_t)BS : n;
-    const uint64_t head = full ? x : x & ((1ull << sh) - 1);
-    const uint32_t glen = full ? 0 : any ? hb + m + 2 : 1;
-    n = any ? bl : n;
-    if (hlen + glen <= 64) {  // both pieces in one word (most planes)
-      const uint32_t len = hlen + glen;
-      const uint64_t code = head | (glen ? grp << (hlen & 63) : 0);
-      const uint32_t l = len < bits ? len : bits;
-      w.put(code & lowmask64(l), l);
-      bits -= l;
+    if constexpr (CUT) {
+      if (len > bits) {
+        len = bits;
+        code &= lowmask64(len);
+      }
     } else {
-      uint32_t l = hlen < bits ? hlen : bits;
-      w.put(head & lowmask64(l), l);
-      bits -= l;
-      l = glen < bits ? glen : bits;
-      w.put(grp & lowmask64(l), l);
-      bits -= l;
+      len = umin(len, bits);
+      code &= lowmask64(len);
     }
+    w.put(code, len);
+    bits -= len;
   }
   return k;
 }
@@ -822,22 +834,31 @@ inline const GroupTable* group_table_host() {
   return &t;
 }
 
-// Planes k, ... down to k_low of a 4^3 block while budget
-// remains, as one flat sequence of steps (a warp's lanes step together
-// whatever plane they are in).  A step takes a plane's verbatim bits and 9
-// bits of its group tests, or 9 more of these.  Close to the last position,
-// whose one is implied, a step takes one group instead; and the token that
-// the budget ends in goes as decode_ints does it (Z/src/template/
-// decode.c:73-105), in a loop of its own that the lanes come to together.
-// Used for 4^3 blocks of 64-bit values: 512^3 doubles at rate 16 decode in
-// 903 us, with a step per token (uncode_flat64, a step per plane and per one)
-// in 996: 300 against 352 warp instructions per block, 29.3 against 26.6 of 32
-// lanes busy.  Other blocks have fewer planes to pay for the longer step and
-// for the table: 3D f32 383 x 385 x 301 at rate 8 168 against 153 us, 2D f32
-// 4093 x 4095 at rate 12 the same, 64^3 floats 17.7 against 15.7.
+// Planes k, ... down to k_low of a 4^3 block while budget remains, as one
+// flat sequence of steps (a warp's lanes step together whatever plane they are
+// in).  A step takes a plane's verbatim bits and 9 bits of its group tests, or
+// 9 more of these.  Close to the last position, whose one is implied, a step
+// takes one group instead; and the token that the budget ends in goes as
+// decode_ints does it (Z/src/template/decode.c:73-105), in a loop of its own
+// that the lanes come to together.
+// (A step per token, that is per plane and per one, with 26.6 of 32 lanes
+// busy, made 352 warp instructions per 4^3 double block at rate 16.)
+// Decoding 320^3 fields, against uncode_flat64 (a step per token) with the
+// whole low slice folded in at once: doubles, smooth, rates 8, 16, 32: 152,
+// 186, 254 against 180, 231, 304 us; noisy 152, 172, 237 against 164, 184,
+// 259; floats, smooth 93, 122, 157 against 126, 156, 202; noisy 96, 116, 161
+// against 102, 118, 161; 64^3 floats 12.3 against 14.2.  Noisy 64-bit
+// integers at high rates, most of whose planes are 64 verbatim bits, are
+// better off with the shorter step of uncode_flat64 (rate 32 246 against 261
+// us, though smooth 292 against 262), so integers above 1024 bits per block
+// take that.  2D blocks, after their runs, have fewer planes to pay for the
+// longer step and the table: f32 4096^2, rate 12, smooth 127 against 125 us,
+// noisy 107 against 95.
 template <int D, typename T>
-GZ_CX bool uses_group_table() { return D == 3 && sizeof(T) == 8; }
-template <class R, class StoreFn>
+GZ_CX bool uses_group_table() { return D == 3; }
+constexpr uint32_t kGroupsMaxIntBits = 1024;
+
+template <int BS, class R, class StoreFn>
 GZ_HD int uncode_groups(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, const GroupTable& t,
                         StoreFn&& store) {
   uint64_t x = 0;       // the plane being built
@@ -852,52 +873,47 @@ GZ_HD int uncode_groups(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, con
     grp = run = false;
   };
   while (k >= k_low && bits) {
-    const uint64_t w = r.peek64();
-    const uint32_t wl = lo32(w), wh = hi32(w);
     const uint32_t h = grp ? 0 : n;
-    // 32 bits from the tests on (fewer, then zeros, for h > 32)
-    const uint32_t g = h < 32 ? fshr(wl, wh, h & 31) : wh >> (h & 31);
+    if (h > bits) break;
+    x |= r.peek64() & lowmask64(h);
+    r.skip(h);
+    bits -= h;
+    grp = true;
+    const uint32_t g = lo32(r.peek64());
     const uint32_t e = t.e[(g & 511u) | (run ? 512u : 0u)];
     uint32_t c = e & 15u, adv = (e >> 4) & 15u, ones = e >> 16;
     bool end = (e >> 8) & 1u, in = (e >> 9) & 1u;
-    if (pos + adv >= 63u || h > 53) {
-      if (h > 53) {  // verbatim bits only
+    if (pos + adv >= BS - 1u) {
+      if (pos == (uint32_t)BS) {  // every coefficient significant: no tests
         c = adv = ones = 0;
-        end = h == 64;
+        end = true;
       } else if (run || (g & 1)) {  // one group, at most 9 positions from the last
-        const uint32_t test = run ? 0u : 1u, z0 = ctz32(g >> test), lim = 63 - pos;
+        const uint32_t test = run ? 0u : 1u, z0 = ctz32(g >> test), lim = BS - 1 - pos;
         const uint32_t z = umin(z0, lim);
         ones = 1u << (z & 31);
         adv = z + 1;
         c = test + z + (z0 < lim ? 1u : 0u);
-        end = pos + adv == 64;
+        end = pos + adv == (uint32_t)BS;
       }
       in = false;
     }
-    if (h + c > bits) break;
-    x |= (w & lowmask64(h)) | ((uint64_t)ones << (pos & 63));
-    c += h;
+    if (c > bits) break;
+    x |= (uint64_t)ones << (pos & 63);
     r.skip(c);
     bits -= c;
     pos += adv;
-    grp = true;
     run = in;
-    if (end) {
-      ends();
-    } else if (!bits) {  // a run cut off by the budget still deposits a one
-      if (run) x |= 1ull << (pos & 63);
-      ends();
-    }
+    if (end) ends();
   }
-  // the budget ends inside the next token
-  while (k >= k_low && bits) {
+  // the budget ends inside the next token, or between two of a plane
+  while (k >= k_low && (bits || grp)) {
     if (!grp) {  // verbatim bits
       const uint32_t h = umin(n, bits);
       x = r.peek64() & lowmask64(h);
       r.skip(h);
       bits -= h;
       grp = true;
-    } else {  // a test and, if it is 1, its group
+    } else if (bits || run) {  // a test and, if it is 1, its group
       uint64_t w = r.peek64();
       if (!run) {
         bits--;
@@ -908,7 +924,8 @@ GZ_HD int uncode_groups(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, con
         }
         w >>= 1;
       }
-      const uint32_t z = ctz64(w), lim = umin(63 - pos, bits);
+      // (a run cut off by the budget still deposits a one)
+      const uint32_t z = ctz64(w), lim = umin(BS - 1 - pos, bits);
       const bool read = z < lim;
       const uint32_t adv = read ? z : lim;
       r.skip(adv + (read ? 1u : 0u));
@@ -917,7 +934,7 @@ GZ_HD int uncode_groups(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, con
       pos += adv + 1;
       run = false;
     }
-    if (pos >= 64 || !bits) ends();
+    if (pos >= (uint32_t)BS || !bits) ends();
   }
   return k;
 }
@@ -1643,6 +1660,21 @@ GZ_HD void planes_to_store(const UInt* u, PS& ps) {
   for (int kk = 0; kk < 32; kk++) ps.put(kk, (uint64_t)t[kk] | ((uint64_t)t[32 + kk] << 32));
 }
 
+// The same for 16 planes: 32G + 16H .. 32G + 16H + 15 into slots 0..15.
+template <int H, class PS>
+GZ_HD void planes16_to_store(const uint32_t* u, PS& ps) {
+  uint32_t t[32];
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      t[16 * h + i] = perm_bytes(u[32 * h + i], u[32 * h + 16 + i], H ? 0x7632 : 0x5410);
+  transpose_tiles<16>(t);
+  transpose_tiles<16>(t + 16);
+#pragma unroll
+  for (int kk = 0; kk < 16; kk++) ps.put(kk, (uint64_t)t[kk] | ((uint64_t)t[16 + kk] << 32));
+}
+
 // Inverse of planes_to_store: slots base + kk for kk in (lo, hi] hold planes
 // 32G + kk, the others are zero; OR the slice into the coefficients.
 // The low and high 32 bits of the planes (coefficients 0..31 and 32..63)
@@ -1659,6 +1691,29 @@ GZ_HD void store_to_coeffs(const PS& ps, int base, int lo, int hi, UInt* u) {
 #pragma unroll
     for (int i = 0; i < 32; i++) u[32 * h + i] |= (UInt)((uint64_t)t[i] << (32 * G));
   }
+}
+
+// Inverse of planes16_to_store: slots kk for kk in (lo, hi] hold planes 16H + kk
+// of the low slice.
+template <int H, class PS>
+GZ_HD void store16_to_coeffs(const PS& ps, int lo, int hi, uint64_t* u) {
+  uint32_t t[32];
+#pragma unroll
+  for (int kk = 0; kk < 16; kk++) {
+    const uint64_t x = (kk > lo && kk <= hi) ? ps.get(kk) : 0;
+    t[kk] = lo32(x);
+    t[16 + kk] = hi32(x);
+  }
+  transpose_tiles<16>(t);
+  transpose_tiles<16>(t + 16);
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t v = t[16 * h + i];
+      u[32 * h + i] |= H ? v << 16 : v & 0xffffu;
+      u[32 * h + 16 + i] |= H ? v & 0xffff0000u : v >> 16;
+    }
 }
 
 // ------------------------------------------------------------- block codec
@@ -1810,13 +1865,27 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
     planes_to_store<1>(u, ps);
     k = code_planes<BS>(k, kmin > 32 ? kmin : 32, n, bits, w,
                         [&](int kk) { return ps.get(kk - 32); });
-    if (k >= kmin && bits) {
+    if constexpr (!F::INT) {
+      // doubles: the low slice 16 planes at a time.  At moderate rates no lane
+      // of a warp needs the last 16, which halves the slice's transposes
+      // (320^3 at rate 16 202 -> 200 us, rate 32 264 -> 259, noisy 276 -> 264;
+      // rate 8 162 -> 163; integers lose about 1%)
+      if (k >= kmin && bits) {
+        planes16_to_store<1>(lo, ps);
+        k = code_planes<BS>(k, kmin > 16 ? kmin : 16, n, bits, w,
+                            [&](int kk) { return ps.get(kk - 16); });
+      }
+      if (k >= kmin && bits) {
+        planes16_to_store<0>(lo, ps);
+        code_planes<BS>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
+      }
+    } else if (k >= kmin && bits) {
       planes_to_store<0>(lo, ps);
       code_planes<BS>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
     }
   } else if constexpr (BS == 64) {
     planes_to_store<0>(u, ps);
-    code_planes<BS>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
+    code_planes<BS, true>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
   } else if constexpr (D == 1) {
     BitString<NW> code;
     uint32_t len = code_planes_4(u, (uint32_t)(P - kmin), *ps.t4, code);
@@ -1934,20 +2003,31 @@ GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* r
     for (int i = 0; i < BS; i++) u[i] = 0;
     if constexpr (P == 64) {
       // top-half planes into the store, folded into the coefficients before
-      // the bottom half reuses the store
+      // the bottom half reuses the store, 16 planes at a time, as it is coded
+      auto planes = [&](int low, int base) {
+        auto store = [&](int kk, uint64_t x) { ps.put(kk - base, x); };
+        if (F::INT && maxbits > kGroupsMaxIntBits)
+          k = uncode_flat64(k, kmin > low ? kmin : low, n, bits, r, store);
+        else
+          k = uncode_groups<BS>(k, kmin > low ? kmin : low, n, bits, r, *ps.gt, store);
+      };
       const int top = k;
-      k = uncode_groups(k, kmin > 32 ? kmin : 32, n, bits, r, *ps.gt,
-                            [&](int kk, uint64_t x) { ps.put(kk - 32, x); });
+      planes(32, 32);
       store_to_coeffs<1>(ps, 0, k - 32, top - 32, u);
       if (k >= kmin && bits) {
+        const int top1 = k;
+        planes(16, 16);
+        store16_to_coeffs<1>(ps, k - 16, top1 - 16, u);
+      }
+      if (k >= kmin && bits) {
         const int top0 = k;
-        k = uncode_groups(k, kmin, n, bits, r, *ps.gt,
-                              [&](int kk, uint64_t x) { ps.put(kk, x); });
-        store_to_coeffs<0>(ps, 0, k, top0, u);
+        planes(0, 0);
+        store16_to_coeffs<0>(ps, k, top0, u);
       }
     } else {
       const int top = k;
-      k = uncode_flat64(k, kmin, n, bits, r, [&](int kk, uint64_t x) { ps.put(kk, x); });
+      k = uncode_groups<BS>(k, kmin, n, bits, r, *ps.gt,
+                            [&](int kk, uint64_t x) { ps.put(kk, x); });
       store_to_coeffs<0>(ps, 0, k, top, u);
     }
   } else if constexpr (D == 1) {

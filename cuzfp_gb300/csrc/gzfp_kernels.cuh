@@ -53,8 +53,7 @@ inline size_t smem_bytes(int slots, int stage, uint32_t maxbits, int tables = 0)
 }
 
 // Tables that a coder's CTAs copy into the start of their shared memory: the
-// 4-value plane tables (1D, 1.6 KB) and the group table (4^3 decoders of
-// 64-bit values, 4 KB).
+// 4-value plane tables (1D, 1.6 KB) and the group table (4^3 decoders, 4 KB).
 struct Tables {
   const Plane4Tables* t4;
   const GroupTable* gt;
