@@ -51,41 +51,105 @@ __device__ __forceinline__ void clear_slot_edges(uint64_t* words, uint64_t pos, 
     atomicAnd((unsigned long long*)(words + w1), (unsigned long long)~lowmask64(hi));
 }
 
-template <int D, typename T>
+// Copy the whole words of a warp's listed slots (lane t's starts at word
+// `first`, if `on`) between the stream and the staged buffer (word j of lane t
+// at buf[j * kStride + t]), 32 consecutive words or so at a time.
+template <bool TO_GLOBAL>
+__device__ __forceinline__ void slots_copy(uint64_t* buf, uint64_t* words, uint64_t first, bool on,
+                                           uint32_t W, uint32_t bpw) {
+  const uint32_t lane = threadIdx.x & 31, total = bpw * W;
+  uint32_t t = lane / W, j = lane % W;
+  const uint32_t dt = 32 / W, dj = 32 % W;
+  const uint32_t act = __ballot_sync(0xffffffffu, on);
+  for (uint32_t e = lane; e - lane < total; e += 32) {
+    const uint32_t src = t < 32 ? t : 0;
+    const uint32_t f0 = __shfl_sync(0xffffffffu, lo32(first), src);
+    const uint32_t f1 = __shfl_sync(0xffffffffu, hi32(first), src);
+    if (e < total && (act >> src & 1)) {
+      uint64_t* g = words + (((uint64_t)f1 << 32) | f0) + j;
+      if (TO_GLOBAL)
+        *g = buf[j * kStride + t];
+      else
+        buf[j * kStride + t] = __ldg(g);
+    }
+    t += dt;
+    j += dj;
+    if (j >= W) {
+      j -= W;
+      t++;
+    }
+  }
+}
+
+// STAGED: slots of whole words, up to kMaxStagedOut of them, go through
+// shared memory, so that a warp reads or writes its slots' words with
+// coalesced accesses instead of one dependent access per lane and word
+// (3D f64, rate 16, read and written: 20,000 blocks 53.7 -> 49.7 us, 2,000
+// blocks 40.5 -> 36.9; f32 42.4 -> 39.7, 28.7 -> 25.6).
+template <int D, typename T, bool STAGED>
 __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
     encode_blocks_kernel(const T* __restrict__ tiles, const unsigned long long* __restrict__ index,
                          const uint8_t* __restrict__ shape, uint64_t count, uint32_t maxbits,
-                         uint64_t* __restrict__ out, uint64_t nwords, uint32_t vec) {
+                         uint64_t* __restrict__ out, uint64_t nwords, uint32_t bpw, uint32_t vec) {
   extern __shared__ __align__(16) uint64_t smem[];
   const Tables tables = stage_tables<D, T, false, kThreads>(smem);
   tables_ready<D, T, false>();
-  SmemPlanes ps{smem + table_words<D, T, false>() + threadIdx.x, tables};
-  const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (i >= count) return;
-  const uint64_t slot = index[i];
-  if (slot >= nwords * 64 / maxbits) return;  // slots past the stream are skipped
+  uint64_t* planes = smem + table_words<D, T, false>();
+  SmemPlanes ps{planes + threadIdx.x, tables};
+  const uint64_t i = lane_block(warp_first_block(bpw), bpw);
+  const uint64_t slot = i < count ? index[i] : ~0ull;
+  const bool on = slot < nwords * 64 / maxbits;  // slots past the stream are skipped
   const uint64_t pos = slot * maxbits;
-  clear_slot_edges(out, pos, maxbits);
-  const Geom g = tile_geom<D>(shape ? shape[i] : 0u, pos, vec);
-  encode_one<D, T>(tiles + i * (1u << (2 * D)), g, 0, maxbits, DevWords{out, nullptr, nwords}, ps);
+  const Geom g = tile_geom<D>(on && shape ? shape[i] : 0u, pos, vec);
+  const T* tile = tiles + i * (1u << (2 * D));
+  if constexpr (STAGED) {
+    const uint32_t W = maxbits >> 6;
+    uint64_t* buf = planes + store_slots<D, T>() * kThreads;
+    if (on)
+      encode_one<D, T, true>(tile, g, 0, maxbits,
+                             StagedWords<kStride>{buf + threadIdx.x, slot * W, W}, ps);
+    __syncwarp();
+    slots_copy<true>(buf + (threadIdx.x & ~31u), out, slot * W, on, W, bpw);
+  } else if (on) {
+    clear_slot_edges(out, pos, maxbits);
+    encode_one<D, T>(tile, g, 0, maxbits, DevWords{out, nullptr, nwords}, ps);
+  }
 }
 
-template <int D, typename T>
+template <int D, typename T, bool STAGED>
 __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
     decode_blocks_kernel(const uint64_t* __restrict__ in, uint64_t nwords,
                          const unsigned long long* __restrict__ index,
                          const uint8_t* __restrict__ shape, uint64_t count, uint32_t maxbits,
-                         T* __restrict__ tiles, uint32_t vec) {
+                         T* __restrict__ tiles, uint32_t bpw, uint32_t vec) {
   extern __shared__ __align__(16) uint64_t smem[];
   const Tables tables = stage_tables<D, T, true, kThreads>(smem);
-  tables_ready<D, T, true>();
-  SmemPlanes ps{smem + table_words<D, T, true>() + threadIdx.x, tables};
-  const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (i >= count) return;
-  const uint64_t slot = index[i];
-  if (slot >= nwords * 64 / maxbits) return;  // slots past the stream are skipped
-  const Geom g = tile_geom<D>(shape ? shape[i] : 0u, slot * maxbits, vec);
-  decode_one<D, T>(tiles + i * (1u << (2 * D)), g, 0, maxbits, DevWords{nullptr, in, nwords}, ps);
+  uint64_t* planes = smem + table_words<D, T, true>();
+  SmemPlanes ps{planes + threadIdx.x, tables};
+  const uint64_t i = lane_block(warp_first_block(bpw), bpw);
+  const uint64_t slot = i < count ? index[i] : ~0ull;
+  const bool on = slot < nwords * 64 / maxbits;  // slots past the stream are skipped
+  const Geom g = tile_geom<D>(on && shape ? shape[i] : 0u, slot * maxbits, vec);
+  T* tile = tiles + i * (1u << (2 * D));
+  if constexpr (STAGED) {
+    const uint32_t W = maxbits >> 6;
+    uint64_t* buf = planes + decode_slots<D, T>() * kThreads;
+    slots_copy<false>(buf + (threadIdx.x & ~31u), (uint64_t*)in, slot * W, on, W, bpw);
+#pragma unroll
+    for (uint32_t j = 0; j < kPadRows; j++) buf[(W + j) * kStride + threadIdx.x] = 0;
+    __syncwarp();
+    tables_ready<D, T, true>();
+    if (on)
+      decode_one<D, T>(tile, g, 0, maxbits,
+                       StagedWords<kStride>{buf + threadIdx.x, slot * W, W}, ps);
+  } else {
+    tables_ready<D, T, true>();
+    if (on) decode_one<D, T>(tile, g, 0, maxbits, DevWords{nullptr, in, nwords}, ps);
+  }
+}
+
+inline int blocks_stage(uint32_t maxbits) {
+  return maxbits % 64 == 0 && maxbits <= 64 * kMaxStagedOut ? kStageRows : kStageNone;
 }
 
 template <int D, typename T>
@@ -93,13 +157,15 @@ cudaError_t launch_encode_blocks_t(const T* tiles, const unsigned long long* ind
                                    const uint8_t* shape, uint64_t count, uint32_t maxbits,
                                    uint64_t* out, uint64_t nwords, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
-  const dim3 grid((unsigned)((count + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(store_slots<D, T>(), kStageNone, 0, table_words<D, T, false>());
-  auto k = encode_blocks_kernel<D, T>;
+  const uint32_t bpw = blocks_per_warp(count, 0);
+  const int stage = blocks_stage(maxbits);
+  const size_t sm = smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D, T, false>());
+  auto k = stage == kStageRows ? encode_blocks_kernel<D, T, true> : encode_blocks_kernel<D, T, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   const uint32_t vec = (uintptr_t)tiles % (4 * sizeof(T)) == 0 ? 1u : 0u;
-  k<<<grid, kThreads, sm, s>>>(tiles, index, shape, count, maxbits, out, nwords, vec);
+  k<<<grid_ctas(count, bpw), kThreads, sm, s>>>(tiles, index, shape, count, maxbits, out, nwords,
+                                               bpw, vec);
   return cudaGetLastError();
 }
 
@@ -108,13 +174,15 @@ cudaError_t launch_decode_blocks_t(const uint64_t* in, uint64_t nwords,
                                    const unsigned long long* index, const uint8_t* shape,
                                    uint64_t count, uint32_t maxbits, T* tiles, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
-  const dim3 grid((unsigned)((count + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0, table_words<D, T, true>());
-  auto k = decode_blocks_kernel<D, T>;
+  const uint32_t bpw = blocks_per_warp(count, 0);
+  const int stage = blocks_stage(maxbits);
+  const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D, T, true>());
+  auto k = stage == kStageRows ? decode_blocks_kernel<D, T, true> : decode_blocks_kernel<D, T, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   const uint32_t vec = (uintptr_t)tiles % (4 * sizeof(T)) == 0 ? 1u : 0u;
-  k<<<grid, kThreads, sm, s>>>(in, nwords, index, shape, count, maxbits, tiles, vec);
+  k<<<grid_ctas(count, bpw), kThreads, sm, s>>>(in, nwords, index, shape, count, maxbits, tiles,
+                                               bpw, vec);
   return cudaGetLastError();
 }
 
