@@ -29,6 +29,7 @@ import ctypes
 import enum
 import math
 import os
+import struct
 from dataclasses import dataclass, field as _dc_field
 from typing import Any, Optional
 
@@ -224,8 +225,10 @@ def zfp_stream_set_accuracy(zfp: zfp_stream, tolerance: float, type: zfp_type) -
 
 def _fixed_rate(zfp: zfp_stream, t: zfp_type) -> bool:
     """The parameters of fixed-rate coding (the fixed-rate path's)."""
-    ints = zfp_type(t) in (zfp_type.int32, zfp_type.int64)
-    prec = 32 if zfp_type(t) in (zfp_type.float, zfp_type.int32) else 64
+    if type(t) is not zfp_type:
+        t = zfp_type(t)
+    ints = t is zfp_type_int32 or t is zfp_type_int64
+    prec = 32 if t is zfp_type_float or t is zfp_type_int32 else 64
     return (zfp.minbits == zfp.maxbits and zfp.maxprec >= prec
             and (ints or zfp.minexp == ZFP_MIN_EXP))
 
@@ -300,8 +303,8 @@ def _cuda_stream_handle(cuda_stream: Any) -> int:
     return int(cuda_stream.cuda_stream)  # torch.cuda.Stream
 
 
-def _check_strided_mode(zfp: zfp_stream, f: zfp_field, strides) -> None:
-    if strides and not _fixed_rate(zfp, f.type):
+def _check_strided_mode(fixed: bool, strides) -> None:
+    if strides and not fixed:
         raise GzfpError(GZFP_ERR_UNSUPPORTED, "strided fields take the fixed-rate path only")
 
 
@@ -316,8 +319,9 @@ def compress(zfp: zfp_stream, f: zfp_field, cuda_stream: Any = None) -> int:
     which returns when the stream is complete.
     """
     strides = _field_strides(f)
-    _check_strided_mode(zfp, f, strides)
-    if not _fixed_rate(zfp, f.type):
+    fixed = _fixed_rate(zfp, f.type)
+    _check_strided_mode(fixed, strides)
+    if not fixed:
         src, _ = _addr_and_size(f.data)
         dst, cap = _addr_and_size(zfp.stream)
         if zfp.capacity is not None:
@@ -353,8 +357,9 @@ def decompress(zfp: zfp_stream, f: zfp_field, cuda_stream: Any = None) -> None:
     src/cuZFP/cuZFP.cu:212-269); in zfp's general mode the blocks are found
     by walking them (see decompress_mode for decoding from known offsets)."""
     strides = _field_strides(f)
-    _check_strided_mode(zfp, f, strides)
-    if not _fixed_rate(zfp, f.type):
+    fixed = _fixed_rate(zfp, f.type)
+    _check_strided_mode(fixed, strides)
+    if not fixed:
         src, size = _addr_and_size(zfp.stream)
         if zfp.capacity is not None:
             size = zfp.capacity
@@ -838,17 +843,36 @@ def default_batch_config() -> BatchConfig:
     return c
 
 
+_BATCH_ITEM = struct.Struct("@iIIIIxxxxPPN")  # gzfp_batch_item
+assert _BATCH_ITEM.size == ctypes.sizeof(BatchItem)
+
+
 def batch_items(fields, streams, rates):
     """ctypes array of gzfp_batch_item for CUDA tensors `fields` (float32 /
     float64 / int32 / int64, 1-3 dims), stream word tensors `streams` and
-    per-array rates."""
-    items = (BatchItem * len(fields))()
-    for i, (f, w, r) in enumerate(zip(fields, streams, rates)):
-        t = _type_of(f.dtype)
-        nx, ny, nz = _dims_of(f.shape)
-        items[i] = BatchItem(int(t), nx, ny, nz,
-                             _lib.gzfp_rate_to_maxbits(int(t), len(f.shape), float(r)),
-                             f.data_ptr(), w.data_ptr(), w.numel() * w.element_size())
+    per-array rates.  (Items are packed as bytes, and each type and each
+    type, rate and dimensionality is looked up once: about 1 us an item,
+    where a structure and the lookups per item took 4.)"""
+    n = len(fields)
+    items = (BatchItem * n)()
+    types, bits = {}, {}
+    pack, size, at = _BATCH_ITEM.pack_into, _BATCH_ITEM.size, 0
+    for f, w, r in zip(fields, streams, rates):
+        dt, shape = f.dtype, f.shape
+        t = types.get(dt)
+        if t is None:
+            t = types[dt] = int(_type_of(dt))
+        d = len(shape)
+        if d == 3:
+            nz, ny, nx = shape
+        else:
+            nx, ny, nz = _dims_of(shape)
+        key = (t, d, r)
+        mb = bits.get(key)
+        if mb is None:
+            mb = bits[key] = _lib.gzfp_rate_to_maxbits(t, d, float(r))
+        pack(items, at, t, nx, ny, nz, mb, f.data_ptr(), w.data_ptr(), w.nbytes)
+        at += size
     return items
 
 

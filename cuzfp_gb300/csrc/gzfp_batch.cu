@@ -214,9 +214,15 @@ using gzfp::bhost::Prepared;
 using gzfp::bhost::valid_config;
 using gzfp::bhost::WorkList;
 
+// The work lists of one device: batches take them in turn, so that a batch is
+// described and queued while the previous ones still run, and waits only for
+// the one that last used its list.  (One list for all held the host up until
+// the previous batch had finished on the device.)
+constexpr int kWorkLists = 4;
 struct DeviceWork {
   std::mutex mu;
-  WorkList wl;
+  WorkList wl[kWorkLists];
+  int next = 0;
 };
 constexpr int kMaxDevices = 64;
 DeviceWork g_work[kMaxDevices];
@@ -238,13 +244,15 @@ int run_batch(const gzfp_batch_item* items, int count, const gzfp_batch_config* 
   cudaStream_t s = (cudaStream_t)cuda_stream;
   DeviceWork& dw = g_work[dev];
   std::lock_guard<std::mutex> lock(dw.mu);
-  // the work list is this device's only one: wait until the previous batch,
-  // on whatever stream it ran, has finished with it
-  if (dw.wl.done && (e = cudaEventSynchronize(dw.wl.done)))
+  WorkList& wl = dw.wl[dw.next];
+  dw.next = (dw.next + 1) % kWorkLists;
+  // wait until the batch that last used this list, on whatever stream it
+  // ran, has finished with it
+  if (wl.done && (e = cudaEventSynchronize(wl.done)))
     return bcuda(e, "cudaEventSynchronize(previous batch)");
-  if ((e = dw.wl.reserve(p.descs.size(), p.lay.nchunks))) return bcuda(e, "batch work list allocation");
-  memcpy(dw.wl.host, p.descs.data(), p.descs.size() * sizeof(gzfp::BatchDesc));
-  if ((e = enqueue(p, dw.wl, decode, cfg, s))) return bcuda(e, "batch launch");
+  if ((e = wl.reserve(p.descs.size(), p.lay.nchunks))) return bcuda(e, "batch work list allocation");
+  memcpy(wl.host, p.descs.data(), p.descs.size() * sizeof(gzfp::BatchDesc));
+  if ((e = enqueue(p, wl, decode, cfg, s))) return bcuda(e, "batch launch");
   return GZFP_OK;
 }
 

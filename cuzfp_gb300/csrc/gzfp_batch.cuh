@@ -270,14 +270,13 @@ cudaError_t launch_batch_kind(int grid, int bpt, bool ahead, uint32_t staged_w,
   const BatchLaunch<NT, DECODE, D, T> L(staged_w);
   cudaError_t e;
   if (grid > 0) {
-    e = cudaFuncSetAttribute(L.persistent, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)L.smem);
+    e = allow_smem(L.persistent, L.smem);
     if (e != cudaSuccess) return e;
     L.persistent<<<grid, NT, L.smem, s>>>(descs, chunk_item, lo, hi, counter, bpt,
                                           ahead ? 1 : 0, L.staged_w);
     return cudaGetLastError();
   }
-  e = cudaFuncSetAttribute(L.grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+  e = allow_smem(L.grid, L.smem);
   if (e != cudaSuccess) return e;
   const uint64_t per = kBatchGridPiece / (uint64_t)bpt;  // chunks per launch
   for (uint64_t c = lo; c < hi; c += per) {

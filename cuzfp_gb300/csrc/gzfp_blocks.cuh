@@ -161,7 +161,7 @@ cudaError_t launch_encode_blocks_t(const T* tiles, const unsigned long long* ind
   const int stage = blocks_stage(maxbits);
   const size_t sm = smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D, T, false>());
   auto k = stage == kStageRows ? encode_blocks_kernel<D, T, true> : encode_blocks_kernel<D, T, false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   const uint32_t vec = (uintptr_t)tiles % (4 * sizeof(T)) == 0 ? 1u : 0u;
   k<<<grid_ctas(count, bpw), kThreads, sm, s>>>(tiles, index, shape, count, maxbits, out, nwords,
@@ -178,7 +178,7 @@ cudaError_t launch_decode_blocks_t(const uint64_t* in, uint64_t nwords,
   const int stage = blocks_stage(maxbits);
   const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D, T, true>());
   auto k = stage == kStageRows ? decode_blocks_kernel<D, T, true> : decode_blocks_kernel<D, T, false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   const uint32_t vec = (uintptr_t)tiles % (4 * sizeof(T)) == 0 ? 1u : 0u;
   k<<<grid_ctas(count, bpw), kThreads, sm, s>>>(in, nwords, index, shape, count, maxbits, tiles,

@@ -286,6 +286,13 @@ inline uint32_t blocks_per_warp(uint64_t nblocks, uint32_t run_bits) {
     bpw /= 2;
   return bpw;
 }
+// Let kernel k have `sm` bytes of dynamic shared memory; up to 47 KB need no
+// leave (48 KB with a kernel's static memory).
+template <class K>
+cudaError_t allow_smem(K k, size_t sm) {
+  if (sm <= 47 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+}
 inline unsigned grid_ctas(uint64_t nblocks, uint32_t bpw) {
   const uint32_t per = kThreads / 32 * bpw;
   return (unsigned)((nblocks + per - 1) / per);
@@ -396,7 +403,7 @@ cudaError_t launch_encode_t(const T* in, const Geom& g, uint32_t maxbits, uint64
   } else if (stage == kStageRows) {
     k = encode_kernel<D, T, kStageRows>;
   }
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   // blocks that share words in place: into a zeroed stream (with a header,
   // the caller has zeroed it and written the header)
@@ -436,7 +443,7 @@ cudaError_t launch_decode_t(const uint64_t* in, uint64_t nwords, const Geom& g, 
     if (stage == kStageRun && maxbits <= 128)
       k = maxbits <= 64 ? decode_kernel<D, T, kStageRun, MB, 1> : decode_kernel<D, T, kStageRun, MB, 2>;
   }
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   const uint32_t bpw = blocks_per_warp(g.nblocks, stage == kStageRun ? maxbits : 0);
   k<<<grid_ctas(g.nblocks, bpw), kThreads, sm, s>>>(in, nwords, g, maxbits, bpw, out);

@@ -106,7 +106,7 @@ cudaError_t launch_encode_mode_t(const T* in, const Geom& g, const General& mode
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
   const size_t sm = smem_bytes(store_slots<D, T>(), kStageNone, 0, table_words<D, T, false>());
   auto k = encode_mode_kernel<D, T>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   k<<<grid, kThreads, sm, s>>>(in, g, mode, scratch, slot_words, lengths);
   return cudaGetLastError();
@@ -120,7 +120,7 @@ cudaError_t launch_decode_mode_t(const uint64_t* in, uint64_t nwords,
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
   const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0, table_words<D, T, true>());
   auto k = decode_mode_kernel<D, T>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   k<<<grid, kThreads, sm, s>>>(in, nwords, offsets, g, mode, out);
   return cudaGetLastError();
