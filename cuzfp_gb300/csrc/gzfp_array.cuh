@@ -165,13 +165,19 @@ GZ_HD void gather(const T* in, const Geom& g, uint32_t ix, uint32_t iy, uint32_t
     for (int z = 0; z < DZ; z++)
 #pragma unroll
       for (int y = 0; y < DY; y++) load_row(base + y * sy + z * sz, raw + 16 * z + 4 * y);
-  } else if (full) {
+  } else if (full && sx == 1) {
+    // rows that are not aligned (nx % 4 != 0): one address a row, not one a
+    // value (3D f32 383 x 385 x 301, rate 8: compress 186 -> 180 us, decompress,
+    // which tested every value's place, 148 -> 146; 3D f64 321 x 320 x 320, rate
+    // 16, compress 246 -> 233)
 #pragma unroll
     for (int z = 0; z < DZ; z++)
 #pragma unroll
-      for (int y = 0; y < DY; y++)
+      for (int y = 0; y < DY; y++) {
+        const T* row = base + y * sy + z * sz;
 #pragma unroll
-        for (int x = 0; x < 4; x++) raw[16 * z + 4 * y + x] = load_bits(base + x * sx + y * sy + z * sz);
+        for (int x = 0; x < 4; x++) raw[16 * z + 4 * y + x] = load_bits(row + x);
+      }
   } else {
 #pragma unroll
     for (int z = 0; z < DZ; z++)
@@ -200,6 +206,17 @@ GZ_HD void scatter(T* out, const Geom& g, uint32_t ix, uint32_t iy, uint32_t iz,
     for (int z = 0; z < DZ; z++)
 #pragma unroll
       for (int y = 0; y < DY; y++) store_row((T*)base + y * sy + z * sz, raw + 16 * z + 4 * y);
+    return;
+  }
+  if (sx == 1 && cx == 4 && (D < 2 || cy == 4) && (D < 3 || cz == 4)) {  // as in gather
+#pragma unroll
+    for (int z = 0; z < DZ; z++)
+#pragma unroll
+      for (int y = 0; y < DY; y++) {
+        UInt* row = base + y * sy + z * sz;
+#pragma unroll
+        for (int x = 0; x < 4; x++) row[x] = raw[16 * z + 4 * y + x];
+      }
     return;
   }
 #pragma unroll

@@ -48,8 +48,8 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
   block_coords(g, b, ix, iy, iz);
   UInt raw[BS];
   gather<D, T>(in, g, ix, iy, iz, raw);
-  BitWriter<DevWords> w(DevWords{scratch + b * slot_words, nullptr, slot_words}, 0,
-                        slot_words * 64);
+  BitWriter<DevWords, true> w(DevWords{scratch + b * slot_words, nullptr, slot_words}, 0,
+                              slot_words * 64);
   lengths[b] = encode_block_mode<D, T>(raw, mode, w, ps);
   w.finish();
 }

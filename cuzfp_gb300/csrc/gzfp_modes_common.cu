@@ -93,31 +93,40 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // Step 3: the len bits of slot b to stream bit offsets[b].  The stream is
 // zeroed first; the words a block shares with its neighbours are merged
-// with atomicOr, the others stored.
+// with atomicOr, the others stored.  A warp places its 32 blocks kPlaceLanes
+// lanes a block, a word each at a time, so that both sides are accessed in
+// runs of consecutive words.  Whole calls, against one lane per block: 256^3
+// doubles at accuracy 1e-6 (11 words a block) 178 -> 167 us, at 28 bits of
+// precision 237 -> 200, 200^3 floats 110 -> 99; with 8 lanes 169, 199 and 101,
+// but small blocks lose (2D f64, 1.5 words a block, 83 -> 85; with 4, 82).
+constexpr int kPlaceLanes = 4;
 __global__ void __launch_bounds__(kThreads)
     place_blocks(const uint64_t* __restrict__ scratch, uint32_t slot_words,
                  const uint32_t* __restrict__ lengths, const uint64_t* __restrict__ offsets,
                  uint64_t nblocks, uint64_t* __restrict__ out) {
-  const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (b >= nblocks) return;
-  const uint32_t len = lengths[b];
-  if (len == 0) return;  // every block takes at least one bit; nothing to place
-  const uint64_t pos = offsets[b], end = pos + len;
-  const uint64_t* src = scratch + b * slot_words;
-  const uint32_t sh = (uint32_t)(pos & 63);
-  const uint32_t nsrc = (len + 63) >> 6;  // source words holding the block
-  const uint64_t w0 = pos >> 6, w1 = (end - 1) >> 6;
-  uint64_t prev = 0;
-  for (uint64_t wi = w0; wi <= w1; wi++) {
-    const uint32_t j = (uint32_t)(wi - w0);
-    const uint64_t cur = j < nsrc ? src[j] : 0;
-    const uint64_t v = sh ? (cur << sh) | (prev >> (64 - sh)) : cur;
-    prev = cur;
-    const bool shared = (wi == w0 && sh) || (wi == w1 && (end & 63));
-    if (shared)
-      atomicOr((unsigned long long*)(out + wi), (unsigned long long)v);
-    else
-      out[wi] = v;
+  constexpr uint32_t kGroups = 32 / kPlaceLanes;
+  const uint32_t lane = threadIdx.x & 31, part = lane % kPlaceLanes, group = lane / kPlaceLanes;
+  const uint64_t b0 = (uint64_t)blockIdx.x * kThreads + (threadIdx.x & ~31u);
+#pragma unroll 2
+  for (uint32_t i = group; i < 32; i += kGroups) {
+    const uint64_t b = b0 + i;
+    if (b >= nblocks) break;
+    const uint32_t len = lengths[b];
+    if (len == 0) continue;  // every block takes at least one bit; nothing to place
+    const uint64_t pos = offsets[b], end = pos + len;
+    const uint64_t* src = scratch + b * slot_words;
+    const uint32_t sh = (uint32_t)(pos & 63);
+    const uint32_t nsrc = (len + 63) >> 6;  // source words holding the block
+    const uint64_t w0 = pos >> 6;
+    const uint32_t last = (uint32_t)(((end - 1) >> 6) - w0);
+    for (uint32_t j = part; j <= last; j += kPlaceLanes) {
+      const uint64_t cur = j < nsrc ? src[j] : 0, prev = j && sh ? src[j - 1] : 0;
+      const uint64_t v = sh ? (cur << sh) | (prev >> (64 - sh)) : cur;
+      if ((j == 0 && sh) || (j == last && (end & 63)))
+        atomicOr((unsigned long long*)(out + w0 + j), (unsigned long long)v);
+      else
+        out[w0 + j] = v;
+    }
   }
 }
 
