@@ -127,6 +127,11 @@ cudaError_t WorkList::reserve(size_t ndesc, size_t nchunks) {
   cudaError_t e = cudaSuccess;
   if (!counter && (e = cudaMalloc(&counter, kBatchKinds * sizeof(unsigned long long)))) return e;
   if (!done && (e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming))) return e;
+  if (!fork && (e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming))) return e;
+  for (int i = 0; i < kSides; i++) {
+    if (!side[i] && (e = cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking))) return e;
+    if (!join[i] && (e = cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming))) return e;
+  }
   if (ndesc > desc_cap) {
     cudaFree(descs);
     cudaFreeHost(host);
@@ -153,6 +158,14 @@ void WorkList::release() {
   cudaFree(chunk_item);
   cudaFree(counter);
   if (done) cudaEventDestroy(done);
+  if (fork) cudaEventDestroy(fork);
+  fork = nullptr;
+  for (int i = 0; i < kSides; i++) {
+    if (side[i]) cudaStreamDestroy(side[i]);
+    if (join[i]) cudaEventDestroy(join[i]);
+    side[i] = nullptr;
+    join[i] = nullptr;
+  }
   descs = nullptr;
   host = nullptr;
   chunk_item = nullptr;
@@ -182,24 +195,49 @@ cudaError_t enqueue(const Prepared& p, WorkList& wl, bool decode, const gzfp_bat
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return e;
   const uint32_t sw = p.lay.staged_w;
   const bool ahead = cfg.claim_ahead != 0;
-  // per kind present, in sequence on the stream: one persistent kernel, or
-  // (ctas_per_sm 0) the grid kernel over the staged items and the grid
-  // kernel over the others
-  for (int k = 0; k < kBatchKinds && !e; k++) {
-    if (p.lay.hi[k] == p.lay.lo[k]) continue;
-    if (cfg.ctas_per_sm == 0) {
-      if (p.lay.mid[k] > p.lay.lo[k])
-        e = launch_batch(cfg.threads, decode, k, 0, cfg.blocks_per_thread, false, sw, wl.descs,
-                         wl.chunk_item, p.lay.lo[k], p.lay.mid[k], wl.counter + k, s);
-      if (!e && p.lay.hi[k] > p.lay.mid[k])
-        e = launch_batch(cfg.threads, decode, k, 0, cfg.blocks_per_thread, false, 0, wl.descs,
-                         wl.chunk_item, p.lay.mid[k], p.lay.hi[k], wl.counter + k, s);
-      continue;
+  if (cfg.ctas_per_sm == 0) {
+    // the grid kernels, two per kind (staged items, the others), largest first
+    // and over up to four streams: most are about a wave of CTAs, and one after
+    // another each would end in a tail that leaves the chip half idle (96 mixed
+    // 3D arrays of 17 to 129 values an edge, compressed and decompressed: 354 ->
+    // 307 us)
+    struct Part {
+      uint64_t lo, hi;
+      int kind;
+      uint32_t sw;
+    };
+    Part part[2 * kBatchKinds];
+    int n = 0;
+    for (int k = 0; k < kBatchKinds; k++) {
+      if (p.lay.mid[k] > p.lay.lo[k]) part[n++] = Part{p.lay.lo[k], p.lay.mid[k], k, sw};
+      if (p.lay.hi[k] > p.lay.mid[k]) part[n++] = Part{p.lay.mid[k], p.lay.hi[k], k, 0};
     }
-    const int grid =
-        sms * std::min(cfg.ctas_per_sm, std::max(1, batch_occupancy(cfg.threads, decode, k, sw)));
-    e = launch_batch(cfg.threads, decode, k, grid, cfg.blocks_per_thread, ahead, sw, wl.descs,
-                     wl.chunk_item, p.lay.lo[k], p.lay.hi[k], wl.counter + k, s);
+    std::sort(part, part + n, [](const Part& a, const Part& b) { return a.hi - a.lo > b.hi - b.lo; });
+    const int sides = std::min(n - 1, WorkList::kSides);
+    if (sides > 0 && (e = cudaEventRecord(wl.fork, s))) return e;
+    int open = 0;  // side streams that wait for the fork, so must be joined
+    for (; open < sides && !e; open++)
+      if ((e = cudaStreamWaitEvent(wl.side[open], wl.fork, 0))) break;
+    for (int i = 0; i < n && !e; i++) {
+      const int at = i % (sides + 1);
+      e = launch_batch(cfg.threads, decode, part[i].kind, 0, cfg.blocks_per_thread, false,
+                       part[i].sw, wl.descs, wl.chunk_item, part[i].lo, part[i].hi,
+                       wl.counter + part[i].kind, at ? wl.side[at - 1] : s);
+    }
+    for (int i = 0; i < open; i++) {
+      cudaError_t ej = cudaEventRecord(wl.join[i], wl.side[i]);
+      if (!ej) ej = cudaStreamWaitEvent(s, wl.join[i], 0);
+      if (!e) e = ej;
+    }
+  } else {
+    // per kind present, in sequence on the stream, one persistent kernel
+    for (int k = 0; k < kBatchKinds && !e; k++) {
+      if (p.lay.hi[k] == p.lay.lo[k]) continue;
+      const int grid =
+          sms * std::min(cfg.ctas_per_sm, std::max(1, batch_occupancy(cfg.threads, decode, k, sw)));
+      e = launch_batch(cfg.threads, decode, k, grid, cfg.blocks_per_thread, ahead, sw, wl.descs,
+                       wl.chunk_item, p.lay.lo[k], p.lay.hi[k], wl.counter + k, s);
+    }
   }
   if (e) return e;
   return wl.done ? cudaEventRecord(wl.done, s) : cudaSuccess;

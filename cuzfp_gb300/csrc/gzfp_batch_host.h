@@ -66,6 +66,11 @@ struct WorkList {
   size_t chunk_cap = 0;
   unsigned long long* counter = nullptr;
   cudaEvent_t done = nullptr;
+  // the grid kernels of a batch's kinds run side by side: side streams, the
+  // event that starts them and those that end them
+  static constexpr int kSides = 3;
+  cudaStream_t side[kSides] = {};
+  cudaEvent_t fork = nullptr, join[kSides] = {};
 
   cudaError_t reserve(size_t ndesc, size_t nchunks);
   void release();
