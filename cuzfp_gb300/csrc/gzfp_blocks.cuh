@@ -81,7 +81,7 @@ __device__ __forceinline__ void slots_copy(uint64_t* buf, uint64_t* words, uint6
   }
 }
 
-// STAGED: slots of whole words, up to kMaxStagedOut of them, go through
+// STAGED: slots of whole words (blocks_stage says how many) go through
 // shared memory, so that a warp reads or writes its slots' words with
 // coalesced accesses instead of one dependent access per lane and word
 // (3D f64, rate 16, read and written: 20,000 blocks 53.7 -> 49.7 us, 2,000
@@ -148,8 +148,19 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
   }
 }
 
-inline int blocks_stage(uint32_t maxbits) {
-  return maxbits % 64 == 0 && maxbits <= 64 * kMaxStagedOut ? kStageRows : kStageNone;
+// Words of the longest staged slot.  Encoder: as elsewhere.  Decoder: longer
+// slots too, up to the 32 words of rate 32, where the reads' latency counts for
+// more than the shared memory: 3D f64, read and written, 30,000 blocks at rate
+// 24 69.7 -> 62.4 us, rate 31 77.3 -> 68.5, 200,000 blocks 284 -> 261, 318 ->
+// 288; f32, rate 31, 13,766 blocks 42.8 -> 40.8.  For values of 32 bits in a
+// list that fills the chip several times over, resident warps count for more:
+// 200,000 blocks at rate 31 186 -> 194 us, so those keep reading the stream, as
+// do slots over 32 words (f64, rate 48, 200,000 blocks: 367 -> 401).
+constexpr uint32_t kMaxStagedSlot = 32;
+constexpr uint64_t kLongList = 1u << 16;
+
+inline int blocks_stage(uint32_t maxbits, uint32_t max_words) {
+  return maxbits % 64 == 0 && maxbits <= 64 * max_words ? kStageRows : kStageNone;
 }
 
 template <int D, typename T>
@@ -158,7 +169,7 @@ cudaError_t launch_encode_blocks_t(const T* tiles, const unsigned long long* ind
                                    uint64_t* out, uint64_t nwords, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
   const uint32_t bpw = blocks_per_warp(count, 0);
-  const int stage = blocks_stage(maxbits);
+  const int stage = blocks_stage(maxbits, kMaxStagedOut);
   const size_t sm = smem_bytes(store_slots<D, T>(), stage, maxbits, table_words<D, T, false>());
   auto k = stage == kStageRows ? encode_blocks_kernel<D, T, true> : encode_blocks_kernel<D, T, false>;
   cudaError_t e = allow_smem(k, sm);
@@ -175,7 +186,8 @@ cudaError_t launch_decode_blocks_t(const uint64_t* in, uint64_t nwords,
                                    uint64_t count, uint32_t maxbits, T* tiles, cudaStream_t s) {
   if (count == 0) return cudaSuccess;
   const uint32_t bpw = blocks_per_warp(count, 0);
-  const int stage = blocks_stage(maxbits);
+  const int stage = blocks_stage(
+      maxbits, sizeof(T) == 8 || count <= kLongList ? kMaxStagedSlot : kMaxStagedOut);
   const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D, T, true>());
   auto k = stage == kStageRows ? decode_blocks_kernel<D, T, true> : decode_blocks_kernel<D, T, false>;
   cudaError_t e = allow_smem(k, sm);
