@@ -122,6 +122,7 @@ cudaError_t index_launch(int type, int dims, const uint64_t* in, uint64_t nwords
 // Bits of a stream that one batch of the index covers at most: its table
 // takes two bytes per bit.
 constexpr uint64_t kIndexBatchBits = 1ull << 28;
+constexpr uint32_t kIndexLeastSegments = 64;  // and the shortest batch, when memory is short
 
 // How often the parallel index widens its range of exponents before it
 // leaves the headers for walks.
@@ -161,26 +162,36 @@ cudaError_t parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* wo
   j.seg_bits = 1024;
   while (j.seg_bits < 32768 && (j.seg_bits <= bound || j.seg_bits < 16 * avg)) j.seg_bits *= 2;
   const uint64_t nseg_all = (span + j.seg_bits - 1) / j.seg_bits;
-  const uint32_t per = (uint32_t)std::min<uint64_t>(nseg_all, kIndexBatchBits / j.seg_bits);
-  while ((uint64_t)j.fan * j.fan * j.fan < per) j.fan++;
-  const uint32_t n1 = (per + j.fan - 1) / j.fan, n2 = (n1 + j.fan - 1) / j.fan;
-  // carve the workspace
-  size_t at = 0;
+  uint32_t per = (uint32_t)std::min<uint64_t>(nseg_all, kIndexBatchBits / j.seg_bits);
+  const size_t maps = (size_t)j.win + 1;
+  uint32_t n1, n2;
+  size_t at, a_state, a_count, a_table, a_first, a_exits, a_hops1, a_hops2, a_entry, a_base;
   auto take = [&](size_t bytes) {
     const size_t a = at;
     at += (bytes + 255) / 256 * 256;
     return a;
   };
-  const size_t maps = (size_t)j.win + 1;
-  const size_t a_state = take(sizeof(IndexState)), a_count = take(2 * sizeof(uint32_t)),
-               a_table = take((size_t)per * j.seg_bits * 2), a_first = take(per * (maps + 1) * 4),
-               a_exits = take(per * maps * 4), a_hops1 = take(n1 * maps * sizeof(IndexHop)),
-               a_hops2 = take(n2 * maps * sizeof(IndexHop)),
-               a_entry = take(((size_t)per + n1 + n2) * 4),
-               a_base = take(((size_t)per + n1 + n2) * 8);
-  if ((e = reserve(ms.index, ms.index_cap, at)) ||
-      (e = reserve(ms.offsets, ms.offsets_cap, (size_t)nblocks * 8)))
-    return e;
+  // carve the workspace; where memory is short, for smaller batches
+  for (;; per = (per + 3) / 4) {
+    j.fan = 0;
+    while ((uint64_t)j.fan * j.fan * j.fan < per) j.fan++;
+    n1 = (per + j.fan - 1) / j.fan;
+    n2 = (n1 + j.fan - 1) / j.fan;
+    at = 0;
+    a_state = take(sizeof(IndexState));
+    a_count = take(2 * sizeof(uint32_t));
+    a_table = take((size_t)per * j.seg_bits * 2);
+    a_first = take(per * (maps + 1) * 4);
+    a_exits = take(per * maps * 4);
+    a_hops1 = take(n1 * maps * sizeof(IndexHop));
+    a_hops2 = take(n2 * maps * sizeof(IndexHop));
+    a_entry = take(((size_t)per + n1 + n2) * 4);
+    a_base = take(((size_t)per + n1 + n2) * 8);
+    e = reserve(ms.index, ms.index_cap, at);
+    if (e != cudaErrorMemoryAllocation || per <= kIndexLeastSegments) break;
+    cudaGetLastError();  // tried again with less
+  }
+  if (e || (e = reserve(ms.offsets, ms.offsets_cap, (size_t)nblocks * 8))) return e;
   char* base = (char*)ms.index;
   j.table = (uint16_t*)(base + a_table);
   uint32_t* counters = (uint32_t*)(base + a_count);

@@ -140,8 +140,8 @@ int gzfp_read_header(const void* header, size_t bytes, int* type, unsigned* nx, 
    capacity of `data`).  Pointers may be host or device memory.
    gzfp_decompress_headed takes streams of every mode: a header naming
    fixed precision, fixed accuracy or other parameters (see "general
-   modes" below) is decoded in that mode, its blocks found by the serial
-   walk of gzfp_index_blocks. */
+   modes" below) is decoded in that mode, its blocks found as gzfp_index_blocks
+   finds them. */
 int gzfp_compress_headed(int type, unsigned nx, unsigned ny, unsigned nz, double rate,
                          const void* data, void* stream, size_t capacity, size_t* out_bytes,
                          void* cuda_stream);
@@ -216,8 +216,9 @@ int gzfp_decompress_mode(int type, unsigned nx, unsigned ny, unsigned nz, const 
                          void* data, void* cuda_stream);
 
 /* Every block's start bit in a stream written with `mode` (by zfp or by
-   gzfp_compress_mode), found by one GPU thread walking the blocks in
-   order: its time grows with the number of blocks, not with the GPU. */
+   gzfp_compress_mode).  Found in parallel, with a workspace of up to about
+   1 GB while the call runs; it returns when the offsets are complete.
+   Streams of at most 32 blocks are walked by one thread. */
 int gzfp_index_blocks(int type, unsigned nx, unsigned ny, unsigned nz, const gzfp_mode* mode,
                       const void* stream, size_t bytes, unsigned long long* offsets,
                       void* cuda_stream);
