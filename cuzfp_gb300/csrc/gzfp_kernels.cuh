@@ -426,9 +426,14 @@ cudaError_t launch_decode_t(const uint64_t* in, uint64_t nwords, const Geom& g, 
   constexpr int MB = MinBlocks<D, T>::value;
   int stage = kStageNone;
   if (g.base == 0 && maxbits % 64 == 0 && (maxbits >> 6) <= kMaxStagedWords) stage = kStageRows;
-  // a run's buffer must not cost a resident CTA
+  // A run's buffer must not cost a resident CTA; of 4^3 blocks of 32-bit values
+  // it may cost the fourth, as the group decoder looks into the stream twice a
+  // step (noisy floats 300x301x299 at rates 20.3, 26.93, 31.82: 149, 168, 169
+  // us from device memory, 118, 130, 152 staged; int32 144, 154, 152 and 117,
+  // 125, 148).
+  constexpr int RB = D == 3 && sizeof(T) == 4 ? 3 : MB;
   if (g.base == 0 && (maxbits % 64 != 0 || (D == 1 && maxbits <= 128)) &&
-      (smem_bytes(decode_slots<D, T>(), kStageRun, maxbits, table_words<D, T, true>()) + 1024) * MB <=
+      (smem_bytes(decode_slots<D, T>(), kStageRun, maxbits, table_words<D, T, true>()) + 1024) * RB <=
           227 * 1024)
     stage = kStageRun;
   const size_t sm = smem_bytes(decode_slots<D, T>(), stage, maxbits, table_words<D, T, true>());
