@@ -1803,7 +1803,8 @@ struct General {
 // so only half of the block's coefficients stay in registers.
 //
 // NW: 64-bit words of a 1D block's code that are wanted (all by default; a
-// fixed-rate caller with a smaller budget asks for fewer).
+// fixed-rate caller with a smaller budget asks for fewer; 0: one word, of a
+// budget of at most 32 bits).
 template <int D, typename T, int NW = code4_words<T>(), class Mode, class W, class PS>
 GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mode, W& w,
                                  PS& ps) {
@@ -1887,8 +1888,18 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
     planes_to_store<0>(u, ps);
     code_planes<BS, true>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
   } else if constexpr (D == 1) {
-    BitString<NW> code;
-    uint32_t len = code_planes_4(u, (uint32_t)(P - kmin), *ps.t4, code);
+    BitString<NW ? NW : 1> code;
+    uint32_t len;
+    if constexpr (NW == 0) {
+      // a plane takes a bit at least: the planes past the budget's bits, so
+      // those past the top 32, do not show
+      uint32_t top[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) top[i] = (uint32_t)(u[i] >> (P - 32));
+      len = code_planes_4(top, umin((uint32_t)(P - kmin), bits), *ps.t4, code);
+    } else {
+      len = code_planes_4(u, (uint32_t)(P - kmin), *ps.t4, code);
+    }
     if constexpr (!F::INT) {
       code.push(head, F::EBITS + 1);
       len += F::EBITS + 1;
@@ -1954,7 +1965,7 @@ struct NoSlice {
 
 // SLICED (4^3 floating-point blocks): the values of z slice z go to
 // slice(z, 16 values) as soon as they are final, and raw is not written.
-// NW as for encode_block_mode.
+// NW as for encode_block_mode, but at least 1.
 template <int D, typename T, bool SLICED = false, int NW = code4_words<T>(), class Mode, class R,
           class PS, class SliceFn = NoSlice>
 GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* raw, PS& ps,

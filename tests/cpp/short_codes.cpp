@@ -23,7 +23,7 @@ void go(bool decode, unsigned nx, unsigned maxbits, void* data, uint64_t* words,
   gzfp::LocalPlanes ps;
   for (uint64_t b = 0; b < g.nblocks; b++) {
     if (decode)
-      gzfp::decode_one<1, T, NW>((T*)data, g, b, maxbits, Words{nullptr, words, n}, ps);
+      gzfp::decode_one<1, T, NW ? NW : 1>((T*)data, g, b, maxbits, Words{nullptr, words, n}, ps);
     else
       gzfp::encode_one<1, T, false, NW>((const T*)data, g, b, maxbits, Words{words, nullptr, n}, ps);
   }
@@ -32,6 +32,7 @@ void go(bool decode, unsigned nx, unsigned maxbits, void* data, uint64_t* words,
 template <typename T>
 void go_t(bool decode, int nw, unsigned nx, unsigned maxbits, void* data, uint64_t* words,
           uint64_t n) {
+  if (nw == 0) go<T, 0>(decode, nx, maxbits, data, words, n);  // encoder: up to 32 bits
   if (nw == 1) go<T, 1>(decode, nx, maxbits, data, words, n);
   if (nw == 2) go<T, 2>(decode, nx, maxbits, data, words, n);
 }

@@ -46,8 +46,8 @@ def test_short_codes(short, orc, dt):
     for bits in range(lo, 129):
         s = np.ascontiguousarray(orc.compress(a, bits / 4.0))
         d = orc.decompress(s, a.shape, dt, bits / 4.0)
-        for nw in (1, 2):
-            if bits > 64 * nw:
+        for nw in (0, 1, 2):
+            if bits > (64 * nw or 32):
                 continue
             w = np.zeros(s.size + 1, np.uint64)
             short.sc_code(0, orc.type_code(dt), nw, a.size, bits, a.ctypes.data, w.ctypes.data, s.size)
@@ -61,6 +61,7 @@ def test_short_codes(short, orc, dt):
 @pytest.mark.parametrize("dt", DTYPES)
 @pytest.mark.parametrize("shape,bits", [
     ((4 * 128 - 1,), (13, 48, 64, 65, 127, 129, 200, 257, 520, 1100)),
+    ((4 * 128 + 1,), (12, 16, 20, 21, 32)),
     ((4 * 128 + 5,), (33, 64, 128, 256)), ((2,), (48,)), ((100003,), (48, 100)),
     ((44, 47), (37, 191, 193, 720, 1001, 1100)), ((401, 203), (90,)),
     ((20, 21, 22), (70, 723, 1000, 1023, 1500, 2700, 4100)), ((52, 33, 37), (500,))])
