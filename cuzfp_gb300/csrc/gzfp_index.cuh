@@ -94,8 +94,6 @@ __global__ void __launch_bounds__(kSampleThreads)
 // the window's end, go to the global list that the link kernels start from.
 // Bound by issue: searching takes 40 instructions per 1024 bits, a 4^3 block
 // about 30 steps of 40 instructions.
-// Per chunk 32,768 bits where the stream is long enough: a lane then parses
-// several blocks, and idles less at the end.
 constexpr uint32_t kHeadsRoom = 256 + 1024;  // listed before parsing, one search
 template <int D, typename T>
 __global__ void __launch_bounds__(32)
@@ -249,11 +247,10 @@ cudaError_t launch_index_fill_t(const IndexJob& j, const IndexLists& l, const In
       (e = cudaMemsetAsync(l.next, 0, sizeof(uint32_t), s)))
     return e;
   if (heads) {
-    uint32_t chunk = j.seg_bits;
-    while (chunk < 32768 && (uint64_t)j.nseg * j.seg_bits / chunk > (uint64_t)sms * 32) chunk *= 2;
-    const uint32_t nw = (63 + chunk + j.win + 64) / 64 + 2;
-    const uint64_t chunks = ((uint64_t)j.nseg * j.seg_bits + chunk - 1) / chunk;
-    index_parse_kernel<D, T><<<(unsigned)chunks, 32, (size_t)nw * 8, s>>>(j, l, chunk, nw, st);
+    const IndexStage g = index_parse_stage(j, sms);
+    const uint64_t chunks = ((uint64_t)j.nseg * j.seg_bits + g.bits - 1) / g.bits;
+    index_parse_kernel<D, T><<<(unsigned)chunks, 32, (size_t)g.words * 8, s>>>(j, l, g.bits,
+                                                                               g.words, st);
   } else {
     index_window_kernel<D, T><<<j.nseg, kWindowThreads, 0, s>>>(j, l);
     index_walk_kernel<D, T><<<sms * 16, kWalkThreads, 0, s>>>(j, l);
@@ -267,15 +264,11 @@ template <int D, typename T>
 cudaError_t launch_index_sample_t(const IndexJob& j, IndexState* st, uint64_t avg, int sms,
                                   cudaStream_t s) {
   const uint64_t span = j.nwords * 64 - j.lo;
-  const uint32_t steady = (uint32_t)index_steady<T>();
-  const uint32_t bits = (uint32_t)(avg < 100 ? 256 : avg < 1600 ? avg * 5 / 2 : 4000);
-  const uint32_t block = (uint32_t)(avg < j.win ? avg : j.win);
-  const uint32_t limit = bits + (steady + 1) * block + 256;
-  const uint32_t nw = (limit + j.win + 64) / 64 + 2;
-  const uint64_t places = span / bits + 1, most = 2 * (uint64_t)sms;
+  const IndexStage g = index_sample_stage<T>(avg, j.win);
+  const uint64_t places = span / g.bits + 1, most = 2 * (uint64_t)sms;
   const uint64_t n = places < most ? places : most;
-  index_sample_kernel<D, T><<<(unsigned)n, kSampleThreads, (size_t)nw * 8, s>>>(
-      j, span / 64 / n, bits, limit, nw, st);
+  index_sample_kernel<D, T><<<(unsigned)n, kSampleThreads, (size_t)g.words * 8, s>>>(
+      j, span / 64 / n, g.bits, g.limit, g.words, st);
   return cudaGetLastError();
 }
 

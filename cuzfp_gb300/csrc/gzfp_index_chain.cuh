@@ -181,6 +181,40 @@ struct IndexSampler {
   }
 };
 
+// What a CTA of the sampling and of the parsing kernel stages: the stream's
+// words from the bits it starts blocks at to the last bit that a block begun
+// there is read at (kParseAhead).
+struct IndexStage {
+  uint32_t bits;   // starts are looked for in the first `bits`
+  uint32_t limit;  // and no block beyond `limit` is begun
+  uint32_t words;  // 64-bit words staged
+};
+inline uint32_t index_stage_words(uint32_t limit, uint32_t win) {
+  return (limit + win + kParseAhead) / 64 + 1;
+}
+// avg: the stream's bits per block
+template <typename T>
+IndexStage index_sample_stage(uint64_t avg, uint32_t win) {
+  const uint32_t block = (uint32_t)(avg < win ? avg : win);
+  IndexStage s;
+  s.bits = (uint32_t)(avg < 100 ? 256 : avg < 1600 ? avg * 5 / 2 : 4000);
+  s.limit = s.bits + ((uint32_t)index_steady<T>() + 1) * block + 256;
+  s.words = index_stage_words(s.limit, win);
+  return s;
+}
+// Whole segments, up to 32,768 bits where the stream is long enough: a lane
+// then parses several blocks, and idles less at the end.  (The first word
+// staged begins up to 63 bits before the chunk.)
+inline IndexStage index_parse_stage(const IndexJob& j, int sms) {
+  const uint64_t all = (uint64_t)j.nseg * j.seg_bits;
+  IndexStage s;
+  s.bits = j.seg_bits;
+  while (s.bits < 32768 && all / s.bits > (uint64_t)sms * 32) s.bits *= 2;
+  s.limit = 63 + s.bits;
+  s.words = index_stage_words(s.limit, j.win);
+  return s;
+}
+
 // A walk from any bit to its segment's end, or to where another has been.
 // tick() takes up the block at p if it is in none, makes up to kSteps steps
 // in it and returns false when the walk ends.  (A warp's lanes are at

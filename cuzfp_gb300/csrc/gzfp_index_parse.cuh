@@ -7,18 +7,19 @@
 
 namespace gzfp {
 
-// The exponent field of a floating-point block's header and the planes the
-// block codes.
+// The exponent field of a floating-point block's header, the planes the
+// block codes and the bits it may take.
 template <int D, typename T>
 struct BlockHead {
   uint32_t field;  // emax + EBIAS
   int prec;
+  uint32_t maxbits;
 };
 
 template <int D, typename T>
 GZ_HD BlockHead<D, T> block_head(uint32_t head, const General& mode) {
   typedef FT<T> F;
-  BlockHead<D, T> h{0, F::P};
+  BlockHead<D, T> h{0, F::P, mode.maxbits};
   if constexpr (!F::INT) {
     h.field = (head >> 1) & ((1u << F::EBITS) - 1);
     h.prec = mode.template precision<D, F::P>((int)h.field - F::EBIAS);
@@ -78,14 +79,19 @@ inline const IndexTables* index_tables_host() {
 // plane that brings coefficients.  Once every coefficient is significant the
 // rest of the planes have known lengths, and a budget that ends inside the
 // block just cuts its length (zfp's coder spends the budget to the last bit).
+// No step is begun past the budget's end, so that whatever the bits say,
+// none is read kParseAhead or more bits past the longest block: up to 22 of
+// planes passed, 33 into a group, and 63 more in the two words of a peek.
 // Same lengths as block_bits.
+constexpr uint32_t kParseAhead = 22 + 33 + 63;
 template <int D, typename T, class R>
 struct BlockParse {
   static constexpr uint32_t BS = 1u << (2 * D);
-  uint32_t cur, start, pos, left;  // bits from the job's first; frontier; planes left
+  uint32_t cur, start, end, pos, left;  // bits from the job's first; frontier; planes left
 
   GZ_HD bool begin(uint32_t p, const BlockHead<D, T>& h) {
     start = p;
+    end = p + h.maxbits;
     cur = p;
     if constexpr (!FT<T>::INT) cur += FT<T>::EBITS + 1;
     pos = 0;
@@ -95,6 +101,7 @@ struct BlockParse {
 
   // true when the block is complete
   GZ_HD bool step(const R& r) {
+    if (cur >= end) return true;  // used() cuts the length
     uint32_t w = r.peek32(cur);
     if (!(w & 1)) {  // planes without new coefficients
       const uint32_t m = r.t->plain[umin(pos, 31u)], hit = w & m;
