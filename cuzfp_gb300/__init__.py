@@ -867,10 +867,10 @@ def batch_items(fields, streams, rates):
             nz, ny, nx = shape
         else:
             nx, ny, nz = _dims_of(shape)
-        key = (t, d, r)
+        key = (t, d, float(r))  # any number: a NumPy scalar array, say, has no hash
         mb = bits.get(key)
         if mb is None:
-            mb = bits[key] = _lib.gzfp_rate_to_maxbits(t, d, float(r))
+            mb = bits[key] = _lib.gzfp_rate_to_maxbits(*key)
         pack(items, at, t, nx, ny, nz, mb, f.data_ptr(), w.data_ptr(), w.nbytes)
         at += size
     return items
