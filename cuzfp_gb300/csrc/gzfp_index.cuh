@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(32)
   __shared__ IndexTables tables;
   __shared__ uint16_t heads[kHeadsRoom];
   __shared__ uint32_t s_next;
+  if (index_over(*st)) return;
   const uint32_t lane = threadIdx.x, at0 = blockIdx.x * chunk;
   const uint32_t size = umin(chunk, j.nseg * j.seg_bits - at0), sh = (uint32_t)(j.lo & 63);
   stage_index_tables(&tables, 32);
@@ -176,8 +177,9 @@ __global__ void __launch_bounds__(32)
 // one CTA per segment, one atomic each.
 template <int D, typename T>
 __global__ void __launch_bounds__(kWindowThreads)
-    index_window_kernel(IndexJob j, IndexLists l) {
+    index_window_kernel(IndexJob j, IndexLists l, const IndexState* st) {
   __shared__ uint32_t s_warp[kWindowThreads / 32];
+  if (index_over(*st)) return;
   const uint32_t s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const DevWords in{nullptr, j.in, j.nwords};
   auto is = [&](uint32_t p) {
@@ -214,9 +216,11 @@ __global__ void __launch_bounds__(kWindowThreads)
 // Each lane takes listed bits until none is left and walks from them to the
 // segment's end or to where another walk has been (IndexLane).
 template <int D, typename T>
-__global__ void __launch_bounds__(kWalkThreads) index_walk_kernel(IndexJob j, IndexLists l) {
+__global__ void __launch_bounds__(kWalkThreads)
+    index_walk_kernel(IndexJob j, IndexLists l, const IndexState* st) {
   typedef IndexStreamReader R;
   __shared__ IndexTables tables;
+  if (index_over(*st)) return;
   stage_index_tables(&tables, kWalkThreads);
   __syncthreads();
   const uint32_t n = *l.count;
@@ -241,19 +245,16 @@ __global__ void __launch_bounds__(kWalkThreads) index_walk_kernel(IndexJob j, In
 template <int D, typename T>
 cudaError_t launch_index_fill_t(const IndexJob& j, const IndexLists& l, const IndexState* st,
                                 bool heads, int sms, cudaStream_t s) {
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(j.table, 0, (size_t)j.nseg * j.seg_bits * 2, s)) ||
-      (e = cudaMemsetAsync(l.count, 0, sizeof(uint32_t), s)) ||
-      (e = cudaMemsetAsync(l.next, 0, sizeof(uint32_t), s)))
-    return e;
+  const cudaError_t e = launch_index_zero(j, l, st, sms, s);
+  if (e != cudaSuccess) return e;
   if (heads) {
     const IndexStage g = index_parse_stage(j, sms);
     const uint64_t chunks = ((uint64_t)j.nseg * j.seg_bits + g.bits - 1) / g.bits;
     index_parse_kernel<D, T><<<(unsigned)chunks, 32, (size_t)g.words * 8, s>>>(j, l, g.bits,
                                                                                g.words, st);
   } else {
-    index_window_kernel<D, T><<<j.nseg, kWindowThreads, 0, s>>>(j, l);
-    index_walk_kernel<D, T><<<sms * 16, kWalkThreads, 0, s>>>(j, l);
+    index_window_kernel<D, T><<<j.nseg, kWindowThreads, 0, s>>>(j, l, st);
+    index_walk_kernel<D, T><<<sms * 16, kWalkThreads, 0, s>>>(j, l, st);
   }
   return cudaGetLastError();
 }

@@ -64,6 +64,11 @@ struct IndexState {
   unsigned int field_lo, field_hi;  // exponent fields (lo > hi: none seen)
 };
 
+// The chain is complete or broken: nothing is left to do for the batches that
+// follow (only the link kernels' last two change it, so that a batch's other
+// kernels all see it alike).
+GZ_HD bool index_over(const IndexState& st) { return st.done || st.broken; }
+
 struct IndexHop {  // entry in the next (group of) segment's window, blocks on the way
   uint32_t exit, count;
 };

@@ -90,6 +90,8 @@ cudaError_t launch_index_sample(int dims, const IndexJob& j, IndexState* st, uin
 template <typename T>
 cudaError_t launch_index_fill(int dims, const IndexJob& j, const IndexLists& l,
                               const IndexState* st, bool heads, int sms, cudaStream_t s);
+cudaError_t launch_index_zero(const IndexJob& j, const IndexLists& l, const IndexState* st, int sms,
+                              cudaStream_t s);
 cudaError_t launch_index_link(const IndexJob& j, const IndexLists& lists, const IndexLinks& l,
                               int sms, IndexState* st, unsigned long long* offsets,
                               cudaStream_t s);

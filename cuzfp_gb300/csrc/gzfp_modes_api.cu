@@ -212,6 +212,7 @@ cudaError_t parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* wo
     e = type == GZFP_TYPE_FLOAT ? launch_index_sample<float>(dims, j, dst, avg, sms, s)
                                 : launch_index_sample<double>(dims, j, dst, avg, sms, s);
   if (e) return e;
+  // (batches after the one that ends the chain return at once)
   for (uint64_t s0 = 0; s0 < nseg_all; s0 += per) {
     j.lo = first + s0 * j.seg_bits;
     j.nseg = (uint32_t)std::min<uint64_t>(per, nseg_all - s0);
