@@ -11,6 +11,7 @@
 
 #include "gzfp.h"
 #include "gzfp_host.h"
+#include "gzfp_index_plan.h"
 #include "gzfp_launch.h"
 
 using namespace gzfp_host;
@@ -119,11 +120,6 @@ cudaError_t index_launch(int type, int dims, const uint64_t* in, uint64_t nwords
   }
 }
 
-// Bits of a stream that one batch of the index covers at most: its table
-// takes two bytes per bit.
-constexpr uint64_t kIndexBatchBits = 1ull << 28;
-constexpr uint32_t kIndexLeastSegments = 64;  // and the shortest batch, when memory is short
-
 // How often the parallel index widens its range of exponents before it
 // leaves the headers for walks.
 constexpr int kIndexTries = 6;
@@ -157,65 +153,40 @@ cudaError_t parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* wo
   j.nblocks = nblocks;
   j.zeros = type != GZFP_TYPE_INT32 && type != GZFP_TYPE_INT64 && mode.minbits <= 1;
   j.win = bound;
-  // Segments of about 24 blocks: the link kernels follow a segment's blocks,
-  // and the segments of a group, one dependent load after another.
-  j.seg_bits = 1024;
-  while (j.seg_bits < 32768 && (j.seg_bits <= bound || j.seg_bits < 16 * avg)) j.seg_bits *= 2;
-  const uint64_t nseg_all = (span + j.seg_bits - 1) / j.seg_bits;
-  uint32_t per = (uint32_t)std::min<uint64_t>(nseg_all, kIndexBatchBits / j.seg_bits);
-  const size_t maps = (size_t)j.win + 1;
-  uint32_t n1, n2;
-  size_t at, a_state, a_count, a_table, a_first, a_exits, a_hops1, a_hops2, a_entry, a_base;
-  auto take = [&](size_t bytes) {
-    const size_t a = at;
-    at += (bytes + 255) / 256 * 256;
-    return a;
-  };
-  // carve the workspace; where memory is short, for smaller batches
-  for (;; per = (per + 3) / 4) {
-    j.fan = 0;
-    while ((uint64_t)j.fan * j.fan * j.fan < per) j.fan++;
-    n1 = (per + j.fan - 1) / j.fan;
-    n2 = (n1 + j.fan - 1) / j.fan;
-    at = 0;
-    a_state = take(sizeof(IndexState));
-    a_count = take(2 * sizeof(uint32_t));
-    a_table = take((size_t)per * j.seg_bits * 2);
-    a_first = take(per * (maps + 1) * 4);
-    a_exits = take(per * maps * 4);
-    a_hops1 = take(n1 * maps * sizeof(IndexHop));
-    a_hops2 = take(n2 * maps * sizeof(IndexHop));
-    a_entry = take(((size_t)per + n1 + n2) * 4);
-    a_base = take(((size_t)per + n1 + n2) * 8);
-    e = reserve(ms.index, ms.index_cap, at);
-    if (e != cudaErrorMemoryAllocation || per <= kIndexLeastSegments) break;
-    cudaGetLastError();  // tried again with less
-  }
-  if (e || (e = reserve(ms.offsets, ms.offsets_cap, (size_t)nblocks * 8))) return e;
+  IndexPlan p = index_plan(span, nblocks, bound);
+  j.seg_bits = p.seg_bits;
+  cudaError_t ea = cudaSuccess;
+  index_reserve(p, [&](size_t bytes) {
+    ea = reserve(ms.index, ms.index_cap, bytes);
+    if (ea == cudaErrorMemoryAllocation) cudaGetLastError();  // not the next call's error
+    return ea == cudaErrorMemoryAllocation ? 1 : ea ? 2 : 0;
+  });
+  if (ea || (e = reserve(ms.offsets, ms.offsets_cap, (size_t)nblocks * 8))) return ea ? ea : e;
+  j.fan = p.fan;
   char* base = (char*)ms.index;
-  j.table = (uint16_t*)(base + a_table);
-  uint32_t* counters = (uint32_t*)(base + a_count);
-  const IndexLists lists{(uint32_t*)(base + a_first), counters, counters + 1};
+  j.table = (uint16_t*)(base + p.table);
+  uint32_t* counters = (uint32_t*)(base + p.counters);
+  const IndexLists lists{(uint32_t*)(base + p.first), counters, counters + 1};
   IndexLinks l{};
-  l.exits = (uint32_t*)(base + a_exits);
-  l.hops1 = (IndexHop*)(base + a_hops1);
-  l.hops2 = (IndexHop*)(base + a_hops2);
-  l.entry0 = (uint32_t*)(base + a_entry);
-  l.entry1 = l.entry0 + per;
-  l.entry2 = l.entry1 + n1;
-  l.base0 = (unsigned long long*)(base + a_base);
-  l.base1 = l.base0 + per;
-  l.base2 = l.base1 + n1;
-  IndexState* dst = (IndexState*)(base + a_state);
+  l.exits = (uint32_t*)(base + p.exits);
+  l.hops1 = (IndexHop*)(base + p.hops1);
+  l.hops2 = (IndexHop*)(base + p.hops2);
+  l.entry0 = (uint32_t*)(base + p.entry);
+  l.entry1 = l.entry0 + p.per;
+  l.entry2 = l.entry1 + p.n1;
+  l.base0 = (unsigned long long*)(base + p.base);
+  l.base1 = l.base0 + p.per;
+  l.base2 = l.base1 + p.n1;
+  IndexState* dst = (IndexState*)(base + p.state);
   if ((e = cudaMemcpyAsync(dst, &st, sizeof st, cudaMemcpyHostToDevice, s))) return e;
   if (heads && st.field_lo > st.field_hi)
     e = type == GZFP_TYPE_FLOAT ? launch_index_sample<float>(dims, j, dst, avg, sms, s)
                                 : launch_index_sample<double>(dims, j, dst, avg, sms, s);
   if (e) return e;
   // (batches after the one that ends the chain return at once)
-  for (uint64_t s0 = 0; s0 < nseg_all; s0 += per) {
+  for (uint64_t s0 = 0; s0 < p.nseg; s0 += p.per) {
     j.lo = first + s0 * j.seg_bits;
-    j.nseg = (uint32_t)std::min<uint64_t>(per, nseg_all - s0);
+    j.nseg = (uint32_t)std::min<uint64_t>(p.per, p.nseg - s0);
     l.n1 = (j.nseg + j.fan - 1) / j.fan;
     l.n2 = (l.n1 + j.fan - 1) / j.fan;
     switch (type) {

@@ -216,9 +216,12 @@ int gzfp_decompress_mode(int type, unsigned nx, unsigned ny, unsigned nz, const 
                          void* data, void* cuda_stream);
 
 /* Every block's start bit in a stream written with `mode` (by zfp or by
-   gzfp_compress_mode).  Found in parallel, with a workspace of up to about
-   1 GB while the call runs; it returns when the offsets are complete.
-   Streams of at most 32 blocks are walked by one thread. */
+   gzfp_compress_mode).  Found in parallel, in batches whose workspace takes at
+   most 1 GiB (less where the stream is shorter or the device has no memory for
+   it); like the other device buffers of the general modes, the library keeps
+   it, one per device, until the process ends.  The call returns when the
+   offsets are complete.  Streams of at most 32 blocks are walked by one
+   thread. */
 int gzfp_index_blocks(int type, unsigned nx, unsigned ny, unsigned nz, const gzfp_mode* mode,
                       const void* stream, size_t bytes, unsigned long long* offsets,
                       void* cuda_stream);
