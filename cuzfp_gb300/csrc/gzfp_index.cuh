@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kSampleThreads)
   }
 }
 
-// Step 2, one warp per `chunk` bits (whole segments): their words staged in shared memory, 32 bits a
+// Step 2, one warp per `chunk` bits: their words staged in shared memory, 32 bits a
 // lane searched for headers at a time (index_heads), the headers listed, and
 // each lane parses listed blocks until none is left.  Those in the window, and
 // the window's end, go to the global list that the link kernels start from.
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(32)
     const uint32_t at = take_next(l.count, m);
     if (is) l.first[at] = at0 + p;
   };
-  for (uint32_t q = 0; q < size; q += 32 * j.seg_bits)
+  for (uint32_t q = (0u - at0) & (j.seg_bits - 1); q < size; q += 32 * j.seg_bits)
     list_entry(q + lane * j.seg_bits < size, q + lane * j.seg_bits + j.win);
   list_entry(lane == 0 && at0 == 0, 0);
   BlockParse<D, T, R> parse;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(32)
     if (lane == 0) s_next = 0;
     __syncwarp();
     for (uint32_t i = lane; i - lane < n; i += 32)
-      list_entry(i < n && (heads[i] & (j.seg_bits - 1)) < j.win, i < n ? heads[i] : 0u);
+      list_entry(i < n && ((at0 + heads[i]) & (j.seg_bits - 1)) < j.win, i < n ? heads[i] : 0u);
     bool live = false, more = true;
     for (;;) {
       const uint32_t idle = __ballot_sync(kLaneAll, !live && more);
@@ -259,17 +259,14 @@ cudaError_t launch_index_fill_t(const IndexJob& j, const IndexLists& l, const In
   return cudaGetLastError();
 }
 
-// Sample the stream's exponents into st: 2 places per SM, or as many as
-// there are.
+// Sample the stream's exponents into st.
 template <int D, typename T>
 cudaError_t launch_index_sample_t(const IndexJob& j, IndexState* st, uint64_t avg, int sms,
                                   cudaStream_t s) {
   const uint64_t span = j.nwords * 64 - j.lo;
-  const IndexStage g = index_sample_stage<T>(avg, j.win);
-  const uint64_t places = span / g.bits + 1, most = 2 * (uint64_t)sms;
-  const uint64_t n = places < most ? places : most;
-  index_sample_kernel<D, T><<<(unsigned)n, kSampleThreads, (size_t)g.words * 8, s>>>(
-      j, span / 64 / n, g.bits, g.limit, g.words, st);
+  const IndexPlaces g = index_sample_stage<T>(span, avg, j.win, sms);
+  index_sample_kernel<D, T><<<(unsigned)g.places, kSampleThreads, (size_t)g.words * 8, s>>>(
+      j, span / 64 / g.places, g.bits, g.limit, g.words, st);
   return cudaGetLastError();
 }
 

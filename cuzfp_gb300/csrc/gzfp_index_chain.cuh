@@ -197,23 +197,34 @@ struct IndexStage {
 inline uint32_t index_stage_words(uint32_t limit, uint32_t win) {
   return (limit + win + kParseAhead) / 64 + 1;
 }
-// avg: the stream's bits per block
+// Of the stream's `span` bits: `places` places, 2 per SM where there are as
+// many.  avg: the stream's bits per block.  (A lane searches its bits one after
+// another, a block's parse for each that may be a first one: fewer bits where
+// the places do not overlap anyway.)
+struct IndexPlaces : IndexStage {
+  uint64_t places;
+};
 template <typename T>
-IndexStage index_sample_stage(uint64_t avg, uint32_t win) {
+IndexPlaces index_sample_stage(uint64_t span, uint64_t avg, uint32_t win, int sms) {
   const uint32_t block = (uint32_t)(avg < win ? avg : win);
-  IndexStage s;
+  const uint64_t most = 2 * (uint64_t)sms, each = span / most + 1;
+  IndexPlaces s;
   s.bits = (uint32_t)(avg < 100 ? 256 : avg < 1600 ? avg * 5 / 2 : 4000);
+  if (each < s.bits) s.bits = each < 256 ? 256 : (uint32_t)each;
   s.limit = s.bits + ((uint32_t)index_steady<T>() + 1) * block + 256;
   s.words = index_stage_words(s.limit, win);
+  const uint64_t n = span / s.bits + 1;
+  s.places = n < most ? n : most;
   return s;
 }
-// Whole segments, up to 32,768 bits where the stream is long enough: a lane
-// then parses several blocks, and idles less at the end.  (The first word
+// 256 to 32,768 bits a warp, as many as leave every scheduler 8 warps: a lane
+// of a long stream then parses several blocks, and idles less at the end; of a
+// short stream as few as there can be, one after another.  (The first word
 // staged begins up to 63 bits before the chunk.)
 inline IndexStage index_parse_stage(const IndexJob& j, int sms) {
   const uint64_t all = (uint64_t)j.nseg * j.seg_bits;
   IndexStage s;
-  s.bits = j.seg_bits;
+  s.bits = 256;
   while (s.bits < 32768 && all / s.bits > (uint64_t)sms * 32) s.bits *= 2;
   s.limit = 63 + s.bits;
   s.words = index_stage_words(s.limit, j.win);

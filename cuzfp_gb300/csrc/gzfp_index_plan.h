@@ -53,20 +53,36 @@ inline void index_carve(IndexPlan& p, uint32_t per) {
   p.bytes = at;
 }
 
-// span: the stream's bits (at least 1); win: the longest block, below 32,768.
-inline IndexPlan index_plan(uint64_t span, uint64_t nblocks, uint32_t win) {
+// span: the stream's bits (at least 1); win: the longest block, below 32,768;
+// heads: by headers, not by walks.
+inline IndexPlan index_plan(uint64_t span, uint64_t nblocks, uint32_t win, bool heads) {
   const uint64_t avg = span / nblocks + 1;
   IndexPlan p;
   p.win = win;
   // Segments of about 24 blocks: the link kernels follow a segment's blocks,
-  // and the segments of a group, one dependent load after another.
+  // and the segments of a group, one dependent load after another.  Of a short
+  // stream shorter ones, so that there are some hundred; some dozen where every
+  // bit of a segment's window is walked from (3D i32, 28 bits of precision: 36
+  // blocks 250 -> 115 us, but 4624 blocks in some hundred 402 -> 510).
+  const uint64_t few = heads ? 1024 : 64;
   p.seg_bits = 1024;
-  while (p.seg_bits < 32768 && (p.seg_bits <= win || p.seg_bits < 16 * avg)) p.seg_bits *= 2;
+  while (p.seg_bits < 32768 &&
+         (p.seg_bits <= win || (p.seg_bits < 16 * avg && span / p.seg_bits > few)))
+    p.seg_bits *= 2;
   p.nseg = (span + p.seg_bits - 1) / p.seg_bits;
   uint64_t per = kIndexBatchBits / p.seg_bits;
   index_carve(p, (uint32_t)(p.nseg < per ? p.nseg : per));
   while (p.bytes > kIndexWorkspace) index_carve(p, p.per - (p.per + 15) / 16);
   return p;
+}
+
+// Streams that one thread walks, block after block, in less time than the
+// parallel index's launches take: of up to 32 blocks, or of a few more with few
+// planes and bits (35 1D blocks of 12 planes: floats 85 us, in parallel 96,
+// int32 73, 104; 68: int32 109, 130, but floats, of more bits, 127, 104; 35
+// blocks of int64 with 28 planes 118, 104).  prec: planes of a block at most.
+inline bool index_serially(uint64_t span, uint64_t nblocks, uint32_t prec) {
+  return nblocks <= 32 || (nblocks * prec <= 832 && span <= 2048);
 }
 
 // The workspace by `alloc` (0: had; 1: no memory; other: failed), for batches

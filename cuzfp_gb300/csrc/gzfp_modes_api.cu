@@ -153,7 +153,7 @@ cudaError_t parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* wo
   j.nblocks = nblocks;
   j.zeros = type != GZFP_TYPE_INT32 && type != GZFP_TYPE_INT64 && mode.minbits <= 1;
   j.win = bound;
-  IndexPlan p = index_plan(span, nblocks, bound);
+  IndexPlan p = index_plan(span, nblocks, bound, heads);
   j.seg_bits = p.seg_bits;
   cudaError_t ea = cudaSuccess;
   index_reserve(p, [&](size_t bytes) {
@@ -202,10 +202,6 @@ cudaError_t parallel_index(ModeSpace& ms, int type, int dims, const uint64_t* wo
   return cudaStreamSynchronize(s);
 }
 
-// Streams of up to this many blocks are walked by one thread (about 5 us a
-// 4^3 block), less than the parallel index's launches and latency.
-constexpr uint64_t kSerialIndexBlocks = 32;
-
 // The blocks of a device stream into ms.offsets; *end_bit = the bit after
 // the last block (past the stream when it ends before its blocks).
 // Synchronises `s`.
@@ -227,7 +223,8 @@ int walk_blocks(ModeSpace& ms, int type, int dims, const uint64_t* words, uint64
     end_bit = first + g.nblocks * mode.minbits;
     return GZFP_OK;
   }
-  if (g.nblocks > kSerialIndexBlocks) {
+  if (!gzfp::index_serially(nwords * 64 - std::min(first, nwords * 64), g.nblocks,
+                            std::min(mode.maxprec, precision_bits(type)))) {
     // no headers in integer streams; where zero blocks are padded (minbits
     // > 1, which no mode sets) a header need not start with a 1
     bool heads = type != GZFP_TYPE_INT32 && type != GZFP_TYPE_INT64 && mode.minbits <= 1;

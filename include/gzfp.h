@@ -220,7 +220,7 @@ int gzfp_decompress_mode(int type, unsigned nx, unsigned ny, unsigned nz, const 
    most 1 GiB (less where the stream is shorter or the device has no memory for
    it); like the other device buffers of the general modes, the library keeps
    it, one per device, until the process ends.  The call returns when the
-   offsets are complete.  Streams of at most 32 blocks are walked by one
+   offsets are complete.  Streams of a few dozen blocks are walked by one
    thread. */
 int gzfp_index_blocks(int type, unsigned nx, unsigned ny, unsigned nz, const gzfp_mode* mode,
                       const void* stream, size_t bytes, unsigned long long* offsets,

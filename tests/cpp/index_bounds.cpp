@@ -6,7 +6,7 @@
 
 #include <algorithm>
 
-#include "gzfp_index_chain.cuh"
+#include "gzfp_index_plan.h"
 
 using namespace gzfp;
 
@@ -53,9 +53,9 @@ void run(const General& mode, const uint64_t* in, uint64_t n, uint64_t nblocks, 
   j.lo = 5;  // as behind a header
   const uint64_t span = n * 64 - j.lo, avg = span / nblocks + 1;
   j.win = win;
-  j.seg_bits = 1024;
-  while (j.seg_bits < 32768 && (j.seg_bits <= win || j.seg_bits < 16 * avg)) j.seg_bits *= 2;
-  j.nseg = (uint32_t)((span + j.seg_bits - 1) / j.seg_bits);
+  const IndexPlan plan = index_plan(span, nblocks, win, true);
+  j.seg_bits = plan.seg_bits;
+  j.nseg = (uint32_t)plan.nseg;  // one batch
   const Stream words{in, n};
 
   const IndexStage g = index_parse_stage(j, sms);
@@ -79,11 +79,10 @@ void run(const General& mode, const uint64_t* in, uint64_t n, uint64_t nblocks, 
     }
   }
 
-  const IndexStage s = index_sample_stage<T>(avg, win);
+  const IndexPlaces s = index_sample_stage<T>(span, avg, win, sms);
   const IndexRange open = index_open<D, T>(mode);
-  const uint64_t places = std::min<uint64_t>(span / s.bits + 1, 2ull * sms);
-  for (uint64_t k = 0; k < places; k++) {
-    const Staged r{in, n, (j.lo >> 6) + k * (span / 64 / places), s.words, 0, &c.outside};
+  for (uint64_t k = 0; k < s.places; k++) {
+    const Staged r{in, n, (j.lo >> 6) + k * (span / 64 / s.places), s.words, 0, &c.outside};
     IndexSampler<D, T, Staged> walk;
     for (uint32_t p = 0; p < s.bits; p++) {
       if (!(r.peek32(p) & 1)) continue;

@@ -56,7 +56,7 @@ int main() {
     const uint32_t win = (uint32_t)upto(9, 4200);
     const uint64_t nblocks = upto(33, 4e9), avg = upto(1, 2.0 * win);
     const uint64_t span = nblocks * avg + upto(1, 64);
-    IndexPlan p = index_plan(span, nblocks, win);
+    IndexPlan p = index_plan(span, nblocks, win, i & 1);
     check(p, span);
     // all of a batch's segments, where one is enough, else most of a limit
     CHECK(p.per == p.nseg || (uint64_t)p.per * p.seg_bits > kIndexBatchBits / 2 ||
@@ -79,7 +79,7 @@ int main() {
     else
       CHECK(r == 1 && p.per <= kIndexLeastSegments, "%d %u", r, p.per);
     // another failure is not tried again
-    IndexPlan q = index_plan(span, nblocks, win);
+    IndexPlan q = index_plan(span, nblocks, win, i & 1);
     calls = 0;
     CHECK(index_reserve(q, [&](size_t) { return calls++, 2; }) == 2 && calls == 1, "%d", calls);
   }
