@@ -98,6 +98,6 @@ cudaError_t launch_index_link(const IndexJob& j, const IndexLists& lists, const 
 
 cudaError_t launch_place_blocks(const uint64_t* scratch, uint32_t slot_words,
                                 const uint32_t* lengths, const unsigned long long* offsets,
-                                uint64_t nblocks, uint64_t* out, cudaStream_t s);
+                                uint64_t nblocks, uint64_t bits, uint64_t* out, cudaStream_t s);
 
 }  // namespace gzfp

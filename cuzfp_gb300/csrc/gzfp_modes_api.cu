@@ -387,7 +387,8 @@ int compress_mode_impl(int type, unsigned nx, unsigned ny, unsigned nz, const gz
                                       cudaMemcpyHostToDevice, s))) ||
       (e = gzfp::launch_place_blocks((const uint64_t*)ms.scratch, slot_words,
                                      (const uint32_t*)ms.lengths,
-                                     (const unsigned long long*)ms.offsets, g.nblocks, dstream, s)))
+                                     (const unsigned long long*)ms.offsets, g.nblocks, total,
+                                     dstream, s)))
     st = cuda_fail(e, "block placement");
   if (!st && !dev_stream && (e = cudaMemcpyAsync(stream, dstream, bytes, cudaMemcpyDeviceToHost, s)))
     st = cuda_fail(e, "cudaMemcpyAsync(stream D2H)");

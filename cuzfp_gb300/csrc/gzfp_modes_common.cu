@@ -97,9 +97,13 @@ __global__ void __launch_bounds__(kScanThreads)
 // lanes a block, a word each at a time, so that both sides are accessed in
 // runs of consecutive words.  Whole calls, against one lane per block: 256^3
 // doubles at accuracy 1e-6 (11 words a block) 178 -> 167 us, at 28 bits of
-// precision 237 -> 200, 200^3 floats 110 -> 99; with 8 lanes 169, 199 and 101,
-// but small blocks lose (2D f64, 1.5 words a block, 83 -> 85; with 4, 82).
-constexpr int kPlaceLanes = 4;
+// precision 237 -> 200, 200^3 floats 110 -> 99; with 8 lanes 169, 199 and 101.
+// Blocks of a word or two, those of 1D fields, are one lane's: 2^22 values, 4
+// lanes against one: f32 104-112 us, 98-105; f64, 12 to 28 bits of precision,
+// 118-132, 112-126; int32 102-105, 92-99.  (From two words on, so 2D fields of
+// 12 bits of precision and more, 4 lanes are as fast or faster.)
+constexpr uint64_t kPlaceAlone = 128;  // bits a block, on average
+template <int kPlaceLanes>
 __global__ void __launch_bounds__(kThreads)
     place_blocks(const uint64_t* __restrict__ scratch, uint32_t slot_words,
                  const uint32_t* __restrict__ lengths, const uint64_t* __restrict__ offsets,
@@ -148,9 +152,10 @@ cudaError_t launch_scan_lengths(const uint32_t* lengths, uint64_t n, uint64_t fi
 
 cudaError_t launch_place_blocks(const uint64_t* scratch, uint32_t slot_words,
                                 const uint32_t* lengths, const unsigned long long* offsets,
-                                uint64_t nblocks, uint64_t* out, cudaStream_t s) {
+                                uint64_t nblocks, uint64_t bits, uint64_t* out, cudaStream_t s) {
   if (nblocks == 0) return cudaSuccess;
-  place_blocks<<<(unsigned)((nblocks + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+  auto k = bits / nblocks < kPlaceAlone ? place_blocks<1> : place_blocks<4>;
+  k<<<(unsigned)((nblocks + kThreads - 1) / kThreads), kThreads, 0, s>>>(
       scratch, slot_words, lengths, (const uint64_t*)offsets, nblocks, out);
   return cudaGetLastError();
 }
