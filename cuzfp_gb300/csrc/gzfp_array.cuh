@@ -336,7 +336,7 @@ struct BitReader {
 
 // ------------------------------------------------------- per-block drivers
 
-template <int D, typename T, bool ALIGNED = false, int NW = code4_words<T>(), class Words, class PS>
+template <int D, typename T, bool ALIGNED = false, int NW = kAnyWords, class Words, class PS>
 GZ_HD void encode_one(const T* in, const Geom& g, uint64_t b, uint32_t maxbits, Words words,
                       PS& ps) {
   typedef typename FT<T>::UInt UInt;
@@ -350,7 +350,7 @@ GZ_HD void encode_one(const T* in, const Geom& g, uint64_t b, uint32_t maxbits, 
   w.finish();
 }
 
-template <int D, typename T, int NW = code4_words<T>(), class Words, class PS>
+template <int D, typename T, int NW = kAnyWords, class Words, class PS>
 GZ_HD void decode_one(T* out, const Geom& g, uint64_t b, uint32_t maxbits, Words words, PS& ps) {
   typedef typename FT<T>::UInt UInt;
   constexpr int BS = 1 << (2 * D);

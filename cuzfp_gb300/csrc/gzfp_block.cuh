@@ -1299,6 +1299,27 @@ struct BitString {
 // Words that hold the longest code of a 4-value block: header, planes, tests.
 template <typename T>
 GZ_CX int code4_words() { return sizeof(T) == 4 ? 3 : 5; }
+// The longest code of np planes: 4 bits each, 3 more where one plane brings
+// all coefficients.
+GZ_HD uint32_t code4_bits(uint32_t np) { return 4 * np + 3; }
+
+// Words of code that a 4-value block's coder works with: a number, 0 (one
+// word, of a budget of at most 32 bits), or as many as the mode and its budget
+// need, found when the coder runs (the kernels that know them beforehand are
+// compiled for a number).
+constexpr int kAnyWords = -1;
+template <int N>
+struct Words_ {
+  static constexpr int value = N;
+};
+
+// The largest budget that the encoder codes from its budget's top planes
+// alone (0 words).  Longer ones gain nothing from fewer planes and pay for
+// finding the last (2^24 - 3 values, planes of the budget against all planes:
+// doubles at rates 4, 6, 8 69, 77, 80 and 83, 86, 84 us; floats at rates 4, 5,
+// 5.5, 6 50, 57, 62, 64 and 55, 59, 59, 59).
+template <typename T>
+constexpr uint32_t kShort1D = sizeof(T) == 8 ? 32 : 20;
 
 // The code of the first np planes (from the top) of a 4-value block, its
 // first 64 N bits, put together from its end: every piece is pushed in front
@@ -1802,10 +1823,8 @@ struct General {
 // bottom slice waits in plane-store slots 32..63 while the top one is coded,
 // so only half of the block's coefficients stay in registers.
 //
-// NW: 64-bit words of a 1D block's code that are wanted (all by default; a
-// fixed-rate caller with a smaller budget asks for fewer; 0: one word, of a
-// budget of at most 32 bits).
-template <int D, typename T, int NW = code4_words<T>(), class Mode, class W, class PS>
+// NW: 64-bit words of a 1D block's code that are wanted (kAnyWords).
+template <int D, typename T, int NW = kAnyWords, class Mode, class W, class PS>
 GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mode, W& w,
                                  PS& ps) {
   typedef FT<T> F;
@@ -1888,32 +1907,55 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
     planes_to_store<0>(u, ps);
     code_planes<BS, true>(k, kmin, n, bits, w, [&](int kk) { return ps.get(kk); });
   } else if constexpr (D == 1) {
-    BitString<NW ? NW : 1> code;
-    uint32_t len;
-    if constexpr (NW == 0) {
-      // a plane takes a bit at least: the planes past the budget's bits, so
-      // those past the top 32, do not show
+    const uint32_t np = (uint32_t)(P - kmin);
+    auto put = [&](auto& code, uint32_t len) -> uint32_t {
+      if constexpr (!F::INT) {
+        code.push(head, F::EBITS + 1);
+        len += F::EBITS + 1;
+      }
+      if constexpr (!Mode::kGeneral) {
+        w.put_string(code, maxbits);
+        return maxbits;
+      } else {
+        const uint32_t used = umin(len, maxbits);
+        const uint32_t all = used < mode.minbits ? mode.minbits : used;
+        code.cut(used);
+        w.put_string(code, all);
+        return all;
+      }
+    };
+    auto whole = [&](auto words) -> uint32_t {  // in so many words
+      BitString<decltype(words)::value> code;
+      const uint32_t len = code_planes_4(u, np, *ps.t4, code);
+      return put(code, len);
+    };
+    auto top32 = [&](auto words, uint32_t planes) -> uint32_t {  // of the top 32 planes
       uint32_t top[4];
 #pragma unroll
       for (int i = 0; i < 4; i++) top[i] = (uint32_t)(u[i] >> (P - 32));
-      len = code_planes_4(top, umin((uint32_t)(P - kmin), bits), *ps.t4, code);
-    } else {
-      len = code_planes_4(u, (uint32_t)(P - kmin), *ps.t4, code);
-    }
-    if constexpr (!F::INT) {
-      code.push(head, F::EBITS + 1);
-      len += F::EBITS + 1;
-    }
-    (void)bits;
-    if constexpr (!Mode::kGeneral) {
-      w.put_string(code, maxbits);
-      return maxbits;
-    } else {
-      const uint32_t used = umin(len, maxbits);
-      const uint32_t all = used < mode.minbits ? mode.minbits : used;
-      code.cut(used);
-      w.put_string(code, all);
-      return all;
+      BitString<decltype(words)::value> code;
+      const uint32_t len = code_planes_4(top, planes, *ps.t4, code);
+      return put(code, len);
+    };
+    // 0 words: a plane takes a bit at least, so the planes past the budget's
+    // bits, and with them those past the top 32, do not show
+    if constexpr (NW == 0) return top32(Words_<1>(), umin(np, bits));
+    else if constexpr (NW > 0) return whole(Words_<NW>());
+    else {
+      // Budgets as the staged kernels take them.  Modes that end a block after
+      // a few planes of many: the top ones.  (With every word and plane / as
+      // needed: 2^22 headed doubles at rates 6, 12 47, 47 / 27, 30 us, floats 31,
+      // 31 / 23, 23; 200,000 listed blocks of doubles at rate 8 16.7 / 8.6; 2^22
+      // doubles with 12, 20 bits of precision, the whole call, 112, 121 / 104,
+      // 113.)
+      if constexpr (!Mode::kGeneral) {
+        if (maxbits <= kShort1D<T>) return top32(Words_<1>(), umin(np, bits));
+        if (maxbits <= 64) return whole(Words_<1>());
+        if (maxbits <= 128) return whole(Words_<2>());
+      } else if constexpr (P == 64) {
+        if (np <= 32) return top32(Words_<3>(), np);
+      }
+      return whole(Words_<code4_words<T>()>());
     }
   } else {
     PL pl;
@@ -1949,7 +1991,7 @@ GZ_HD uint32_t encode_block_mode(const typename FT<T>::UInt* raw, const Mode& mo
   }
 }
 
-template <int D, typename T, int NW = code4_words<T>(), class W, class PS>
+template <int D, typename T, int NW = kAnyWords, class W, class PS>
 GZ_HD void encode_block(const typename FT<T>::UInt* raw, uint32_t maxbits, W& w, PS& ps) {
   encode_block_mode<D, T, NW>(raw, FixedRate{maxbits}, w, ps);
 }
@@ -1965,8 +2007,8 @@ struct NoSlice {
 
 // SLICED (4^3 floating-point blocks): the values of z slice z go to
 // slice(z, 16 values) as soon as they are final, and raw is not written.
-// NW as for encode_block_mode, but at least 1.
-template <int D, typename T, bool SLICED = false, int NW = code4_words<T>(), class Mode, class R,
+// NW as for encode_block_mode, but not 0.
+template <int D, typename T, bool SLICED = false, int NW = kAnyWords, class Mode, class R,
           class PS, class SliceFn = NoSlice>
 GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* raw, PS& ps,
                                  SliceFn&& slice = SliceFn{}) {
@@ -2048,16 +2090,34 @@ GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* r
       store_to_coeffs<0>(ps, 0, k, top, u);
     }
   } else if constexpr (D == 1) {
-    BitString<NW> code;
-    uint32_t left = bits;
+    const uint32_t np = (uint32_t)(P - kmin);
+    auto words = [&](auto n, uint32_t left) {  // from the first `left` bits
+      constexpr int N = decltype(n)::value;
+      BitString<N> code;
 #pragma unroll
-    for (int i = 0; i < NW; i++) {
-      const uint32_t c = umin(left, 64u);
-      code.w[i] = c ? r.peek64() & lowmask64(c) : 0;
-      if (i + 1 < NW) r.skip(c);
-      left -= c;
+      for (int i = 0; i < N; i++) {
+        const uint32_t c = umin(left, 64u);
+        code.w[i] = c ? r.peek64() & lowmask64(c) : 0;
+        if (i + 1 < N) r.skip(c);
+        left -= c;
+      }
+      uncode_planes_4(u, np, bits, code, *ps.t4);
+    };
+    if constexpr (NW > 0) {
+      words(Words_<NW>(), bits);
+    } else {
+      // no bits past the planes' longest code, nor words of it (2^22 values:
+      // headed doubles at rates 6, 12 79, 82 -> 68, 70 us; from start bits,
+      // doubles with 12, 20, 28 bits of precision 33, 47, 47 -> 21, 31, 31,
+      // floats 23, 31, 31 -> 17, 27, 27)
+      const uint32_t need = umin(bits, code4_bits(np));
+      if (need <= 64)
+        words(Words_<1>(), need);
+      else if (need <= 128)
+        words(Words_<2>(), need);
+      else
+        words(Words_<code4_words<T>()>(), need);
     }
-    uncode_planes_4(u, (uint32_t)(P - kmin), bits, code, *ps.t4);
   } else {
 #pragma unroll
     for (int i = 0; i < PL::NW; i++) ps.put(i, 0);
@@ -2111,7 +2171,7 @@ GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* r
   return used < mode.min_bits() ? mode.min_bits() : used;
 }
 
-template <int D, typename T, int NW = code4_words<T>(), class R, class PS>
+template <int D, typename T, int NW = kAnyWords, class R, class PS>
 GZ_HD void decode_block(R& r, uint32_t maxbits, typename FT<T>::UInt* raw, PS& ps) {
   decode_block_mode<D, T, false, NW>(r, FixedRate{maxbits}, raw, ps);
 }

@@ -382,14 +382,6 @@ __global__ void __launch_bounds__(kThreads, MINB)
   }
 }
 
-// The largest 1D budget that the encoder codes from its budget's top planes
-// alone (NW = 0).  Longer ones gain nothing from fewer planes and pay for
-// finding the last (2^24 - 3 values, planes of the budget against all planes:
-// doubles at rates 4, 6, 8 69, 77, 80 and 83, 86, 84 us; floats at rates 4, 5,
-// 5.5, 6 50, 57, 62, 64 and 55, 59, 59, 59).
-template <typename T>
-constexpr uint32_t kShort1D = sizeof(T) == 8 ? 32 : 20;
-
 // Kernel launchers shared by the per-type translation units.  The encoder
 // stages blocks of up to kMaxStagedOut words when their buffer fits beside
 // the plane store without costing a resident CTA (larger blocks measured
