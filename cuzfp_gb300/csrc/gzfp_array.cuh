@@ -296,6 +296,16 @@ struct BitWriter {
 };
 
 // ------------------------------------------------------------- bit reader
+// the 64 bits from bit `off` (below 64) of (w1:w0): one funnel shift per
+// result word
+GZ_HD uint64_t window64(uint64_t w0, uint64_t w1, uint32_t off) {
+  const uint32_t a0 = lo32(w0), a1 = hi32(w0), a2 = lo32(w1), a3 = hi32(w1);
+  const bool ge = off >= 32;
+  const uint32_t s = off & 31;
+  const uint32_t b0 = ge ? a1 : a0, b1 = ge ? a2 : a1, b2 = ge ? a3 : a2;
+  return ((uint64_t)fshr(b1, b2, s) << 32) | fshr(b0, b1, s);
+}
+
 template <class Words>
 struct BitReader {
   Words words;
@@ -309,14 +319,7 @@ struct BitReader {
     w0 = words.load(wi);
     w1 = words.load(wi + 1);
   }
-  GZ_HD uint64_t peek64() const {
-    // the 64 bits from `off` of (w1:w0): one funnel shift per result word
-    const uint32_t a0 = lo32(w0), a1 = hi32(w0), a2 = lo32(w1), a3 = hi32(w1);
-    const bool ge = off >= 32;
-    const uint32_t s = off & 31;
-    const uint32_t b0 = ge ? a1 : a0, b1 = ge ? a2 : a1, b2 = ge ? a3 : a2;
-    return ((uint64_t)fshr(b1, b2, s) << 32) | fshr(b0, b1, s);
-  }
+  GZ_HD uint64_t peek64() const { return window64(w0, w1, off); }
   GZ_HD void skip(uint32_t n) {  // n <= 64
     off += n;
     if (off >= 64) {

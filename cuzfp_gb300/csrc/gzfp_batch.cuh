@@ -101,7 +101,7 @@ __device__ __forceinline__ void batch_block(const BatchDesc& d, uint64_t b, Batc
     }
     if (b >= d.g.nblocks) return;
     decode_one<D, T>((T*)d.out, d.g, b, d.maxbits,
-                     DevWords{nullptr, (const uint64_t*)d.in, d.nwords}, ps);
+                     StreamWords<D>{(const uint64_t*)d.in, d.nwords}, ps);
   } else {
     const uint32_t W = d.maxbits >> 6;
     if (PATH == kPathStaged ||

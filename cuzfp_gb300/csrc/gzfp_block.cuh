@@ -857,6 +857,15 @@ inline const GroupTable* group_table_host() {
 template <int D, typename T>
 GZ_CX bool uses_group_table() { return D == 3; }
 constexpr uint32_t kGroupsMaxIntBits = 1024;
+// FixedRate by type and budget; the general modes as the kernel is compiled
+// (GeneralTokens, decode_mode_kernel).
+template <typename T, class Mode>
+GZ_HD bool groups_by_table(const Mode& m) {
+  if constexpr (Mode::kGeneral)
+    return !Mode::kTokens;
+  else
+    return !FT<T>::INT || FT<T>::P == 32 || m.maxbits <= kGroupsMaxIntBits;
+}
 
 template <int BS, class R, class StoreFn>
 GZ_HD int uncode_groups(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, const GroupTable& t,
@@ -1782,7 +1791,7 @@ GZ_HD void front_end_int(const typename FT<T>::UInt* raw, typename FT<T>::UInt* 
 // fixed-rate kernels compile; General holds all four (fixed precision,
 // fixed accuracy, or any setting of zfp_stream_set_params).
 struct FixedRate {
-  static constexpr bool kGeneral = false;
+  static constexpr bool kGeneral = false, kTop32 = false;
   uint32_t maxbits;
   GZ_HD uint32_t min_bits() const { return maxbits; }
   // planes a floating-point block codes: precision() of
@@ -1797,7 +1806,7 @@ struct FixedRate {
 };
 
 struct General {
-  static constexpr bool kGeneral = true;
+  static constexpr bool kGeneral = true, kTokens = false, kTop32 = false;
   uint32_t minbits, maxbits, maxprec;
   int minexp;
   GZ_HD uint32_t min_bits() const { return minbits; }
@@ -1812,6 +1821,13 @@ struct General {
   // lowest plane of an integer block: P - maxprec (Z/src/template/encode.c:127)
   template <int P>
   GZ_HD int int_kmin() const { return (uint32_t)P > maxprec ? P - (int)maxprec : 0; }
+};
+// the same, its 4^3 blocks decoded by token (uncode_flat64); TOP32: of modes
+// with at most 32 planes
+template <bool TOP32>
+struct GeneralTokens : General {
+  static constexpr bool kTokens = true, kTop32 = TOP32;
+  GZ_HD explicit GeneralTokens(const General& g) : General(g) {}
 };
 
 // Encode one block of raw IEEE bit patterns (gathered and padded)
@@ -2059,34 +2075,33 @@ GZ_HD uint32_t decode_block_mode(R& r, const Mode& mode, typename FT<T>::UInt* r
       // the bottom half reuses the store, 16 planes at a time, as it is coded
       auto planes = [&](int low, int base) {
         auto store = [&](int kk, uint64_t x) { ps.put(kk - base, x); };
-        if (F::INT && maxbits > kGroupsMaxIntBits)
-          k = uncode_flat64(k, kmin > low ? kmin : low, n, bits, r, store);
-        else
+        if (groups_by_table<T>(mode))
           k = uncode_groups<BS>(k, kmin > low ? kmin : low, n, bits, r, *ps.gt, store);
+        else
+          k = uncode_flat64(k, kmin > low ? kmin : low, n, bits, r, store);
       };
       const int top = k;
       planes(32, 32);
       store_to_coeffs<1>(ps, 0, k - 32, top - 32, u);
-      if (k >= kmin && bits) {
-        const int top1 = k;
-        planes(16, 16);
-        store16_to_coeffs<1>(ps, k - 16, top1 - 16, u);
-      }
-      if (k >= kmin && bits) {
-        const int top0 = k;
-        planes(0, 0);
-        store16_to_coeffs<0>(ps, k, top0, u);
+      if constexpr (!Mode::kTop32) {
+        if (k >= kmin && bits) {
+          const int top1 = k;
+          planes(16, 16);
+          store16_to_coeffs<1>(ps, k - 16, top1 - 16, u);
+        }
+        if (k >= kmin && bits) {
+          const int top0 = k;
+          planes(0, 0);
+          store16_to_coeffs<0>(ps, k, top0, u);
+        }
       }
     } else {
       const int top = k;
       auto store = [&](int kk, uint64_t x) { ps.put(kk, x); };
-      // int32 in the general modes: its planes are dense from the first ones
-      // on (300^3 from start bits, precision 12, 20, 28: by table 54, 68, 92
-      // us, noisy 54, 68, 118; by token 48, 65, 99, noisy 48, 66, 115)
-      if constexpr (F::INT && Mode::kGeneral)
-        k = uncode_flat64(k, kmin, n, bits, r, store);
-      else
+      if (groups_by_table<T>(mode))
         k = uncode_groups<BS>(k, kmin, n, bits, r, *ps.gt, store);
+      else
+        k = uncode_flat64(k, kmin, n, bits, r, store);
       store_to_coeffs<0>(ps, 0, k, top, u);
     }
   } else if constexpr (D == 1) {

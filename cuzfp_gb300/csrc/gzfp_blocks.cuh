@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
                          const uint8_t* __restrict__ shape, uint64_t count, uint32_t maxbits,
                          T* __restrict__ tiles, uint32_t bpw, uint32_t vec) {
   extern __shared__ __align__(16) uint64_t smem[];
-  const Tables tables = stage_tables<D, T, true, kThreads>(smem);
+  const bool use = D != 3 || groups_by_table<T>(FixedRate{maxbits});
+  const Tables tables = stage_tables<D, T, true, kThreads>(smem, use);
   uint64_t* planes = smem + table_words<D, T, true>();
   SmemPlanes ps{planes + threadIdx.x, tables};
   const uint64_t i = lane_block(warp_first_block(bpw), bpw);
@@ -138,13 +139,13 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
 #pragma unroll
     for (uint32_t j = 0; j < kPadRows; j++) buf[(W + j) * kStride + threadIdx.x] = 0;
     __syncwarp();
-    tables_ready<D, T, true>();
+    tables_ready<D, T, true>(use);
     if (on)
       decode_one<D, T>(tile, g, 0, maxbits,
                        StagedWords<kStride>{buf + threadIdx.x, slot * W, W}, ps);
   } else {
-    tables_ready<D, T, true>();
-    if (on) decode_one<D, T>(tile, g, 0, maxbits, DevWords{nullptr, in, nwords}, ps);
+    tables_ready<D, T, true>(use);
+    if (on) decode_one<D, T>(tile, g, 0, maxbits, StreamWords<D>{in, nwords}, ps);
   }
 }
 

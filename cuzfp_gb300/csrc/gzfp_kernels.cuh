@@ -68,10 +68,10 @@ __host__ __device__ constexpr int table_words() {
 // Start copying the coder's tables into shared memory (16 bytes aligned),
 // and wait for them: the CTA's own staging goes between the two, so that the
 // copies' latencies overlap.  Every thread of the CTA must call both before
-// any thread returns; tables_ready is a CTA barrier where there are tables
-// (and where ALWAYS is set).
+// any thread returns, with the same `use` (is a table looked up at all);
+// tables_ready is a CTA barrier where one is (and where ALWAYS is set).
 template <int D, typename T, bool DECODE, int NT>
-__device__ __forceinline__ Tables stage_tables(uint64_t* smem) {
+__device__ __forceinline__ Tables stage_tables(uint64_t* smem, bool use = true) {
   constexpr int n = table_words<D, T, DECODE>() / 2;  // 16-byte pieces
   if constexpr (n == 0) {
     return Tables{nullptr, nullptr};
@@ -79,24 +79,25 @@ __device__ __forceinline__ Tables stage_tables(uint64_t* smem) {
     const char* src = D == 1 ? reinterpret_cast<const char*>(&kPlane4Tables)
                              : reinterpret_cast<const char*>(&kGroupTable);
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+    if (use) {
 #pragma unroll
-    for (int i = threadIdx.x; i < n; i += NT)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i),
-                   "l"(src + 16 * i) : "memory");
+      for (int i = threadIdx.x; i < n; i += NT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i),
+                     "l"(src + 16 * i) : "memory");
+    }
     return Tables{reinterpret_cast<const Plane4Tables*>(smem),
                   reinterpret_cast<const GroupTable*>(smem)};
   }
 }
 template <int D, typename T, bool DECODE, bool ALWAYS = false>
-__device__ __forceinline__ void tables_ready() {
+__device__ __forceinline__ void tables_ready(bool use = true) {
   if constexpr (table_words<D, T, DECODE>() > 0) {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
+    if (use) asm volatile("cp.async.wait_all;" ::: "memory");
+    if (use || ALWAYS) __syncthreads();
   } else if constexpr (ALWAYS) {
     __syncthreads();
   }
 }
-
 // per-thread plane store in shared memory, slot i at planes[i * kThreads]
 struct SmemPlanes {
   uint64_t* p;
@@ -119,6 +120,23 @@ struct DevWords {
   }
   __device__ __forceinline__ uint64_t load(uint64_t i) const { return i < n ? __ldg(in + i) : 0; }
 };
+
+// Global stream words for reading alone.  4^3 blocks: AHEAD, with a reader that
+// loads the word behind the two that a peek spans before it is needed.  The
+// group decoder looks at the stream up to twice a step, and waited for each new
+// word (300^3, rates 6, 12, 24 behind a header: floats 139, 156, 190 -> 131,
+// 143, 168 us, smooth 143, 168, 194 -> 133, 155, 170; noisy doubles 200, 224, 307
+// -> 193, 205, 265; from start bits, 28 bits of precision, noisy: floats 134 ->
+// 125, doubles 224 -> 190).  By token, with shorter steps, it costs more than it
+// gives (int32 from start bits, precision 20: 58 -> 60).
+template <bool AHEAD>
+struct ReadWords {
+  const uint64_t* in;
+  uint64_t n;
+  __device__ __forceinline__ uint64_t load(uint64_t i) const { return i < n ? __ldg(in + i) : 0; }
+};
+template <int D>
+using StreamWords = ReadWords<D == 3>;
 
 // One block's slot in the staged word buffer: word j of the block at
 // buf[j * PITCH] (PITCH = threads per CTA + 1, so the 32 lanes of a warp
@@ -207,19 +225,46 @@ struct BitReader<StagedWords<PITCH>> {
   __device__ __forceinline__ BitReader(StagedWords<PITCH> w, uint64_t p)
       : buf(w.buf), pos((uint32_t)(p - (w.w0 << 6))) {}
   __device__ __forceinline__ uint64_t peek64() const {
-    const uint32_t j = pos >> 6, s = pos & 63;
-    const uint64_t a = buf[j * PITCH], b = buf[(j + 1) * PITCH];
-    const uint32_t a0 = lo32(a), a1 = hi32(a), b0 = lo32(b), b1 = hi32(b);
-    const bool ge = s >= 32;
-    const uint32_t c0 = ge ? a1 : a0, c1 = ge ? b0 : a1, c2 = ge ? b1 : b0;
-    const uint32_t t = s & 31;
-    return ((uint64_t)__funnelshift_r(c1, c2, t) << 32) | __funnelshift_r(c0, c1, t);
+    const uint32_t j = pos >> 6;
+    return window64(buf[j * PITCH], buf[(j + 1) * PITCH], pos & 63);
   }
   __device__ __forceinline__ void skip(uint32_t n) { pos += n; }
   __device__ __forceinline__ uint64_t read(uint32_t n) {
     if (n == 0) return 0;
     const uint64_t v = peek64() & lowmask64(n);
     pos += n;
+    return v;
+  }
+};
+
+// Bit reader with a word loaded ahead.
+template <>
+struct BitReader<ReadWords<true>> {
+  ReadWords<true> words;
+  uint64_t wi;          // index of w0
+  uint64_t w0, w1, w2;
+  uint32_t off;
+  __device__ __forceinline__ BitReader(ReadWords<true> w, uint64_t pos)
+      : words(w), wi(pos >> 6), off((uint32_t)(pos & 63)) {
+    w0 = words.load(wi);
+    w1 = words.load(wi + 1);
+    w2 = words.load(wi + 2);
+  }
+  __device__ __forceinline__ uint64_t peek64() const { return window64(w0, w1, off); }
+  __device__ __forceinline__ void skip(uint32_t n) {  // n <= 64
+    off += n;
+    if (off >= 64) {
+      off -= 64;
+      wi++;
+      w0 = w1;
+      w1 = w2;
+      w2 = words.load(wi + 2);
+    }
+  }
+  __device__ __forceinline__ uint64_t read(uint32_t n) {
+    if (n == 0) return 0;
+    const uint64_t v = peek64() & lowmask64(n);
+    skip(n);
     return v;
   }
 };
@@ -351,7 +396,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
   extern __shared__ __align__(16) uint64_t smem[];
   uint64_t* buf = smem + table_words<D, T, true>() + decode_slots<D, T>() * kThreads;
   const uint64_t w0 = (uint64_t)blockIdx.x * (bpw * maxbits / 16);
-  const Tables tables = stage_tables<D, T, true, kThreads>(smem);
+  const bool use = D != 3 || groups_by_table<T>(FixedRate{maxbits});
+  const Tables tables = stage_tables<D, T, true, kThreads>(smem, use);
   if constexpr (STAGE == kStageRun) {
     const uint64_t left = nwords - w0;
     for (uint32_t i = threadIdx.x; i < bpw * maxbits / 16 + kPadRows; i += kThreads)
@@ -369,16 +415,16 @@ __global__ void __launch_bounds__(kThreads, MINB)
 #pragma unroll
     for (uint32_t j = 0; j < kPadRows; j++) buf[(W + j) * kStride + threadIdx.x] = 0;
     __syncwarp();
-    tables_ready<D, T, true>();
+    tables_ready<D, T, true>(use);
     if (b < g.nblocks)
       decode_one<D, T>(out, g, b, maxbits, StagedWords<kStride>{buf + threadIdx.x, b * W, W}, ps);
   } else if constexpr (STAGE == kStageRun) {
-    tables_ready<D, T, true, true>();
+    tables_ready<D, T, true, true>(use);
     if (b < g.nblocks)
       decode_one<D, T, NW>(out, g, b, maxbits, StagedWords<1>{buf, w0, bpw * maxbits / 16}, ps);
   } else {
-    tables_ready<D, T, true>();
-    if (b < g.nblocks) decode_one<D, T>(out, g, b, maxbits, DevWords{nullptr, in, nwords}, ps);
+    tables_ready<D, T, true>(use);
+    if (b < g.nblocks) decode_one<D, T>(out, g, b, maxbits, StreamWords<D>{in, nwords}, ps);
   }
 }
 

@@ -57,25 +57,39 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
 // Steps 2 and 3 (the scan of the lengths and the placement of the blocks)
 // do not depend on the scalar type: gzfp_modes_common.cu.
 
+// How general-mode blocks are decoded: with the coder's tables, or 4^3 blocks
+// by token, without the group table and its space; of 64-bit values at most 32
+// planes of them, without the code for the others.
+constexpr int kByTable = 0, kByToken = 1, kByTokenTop32 = 2;
+
 // Decode block b from stream bit offsets[b].
-template <int D, typename T>
+template <int D, typename T, int HOW>
 __global__ void __launch_bounds__(kThreads, (MinBlocks<D, T>::value))
     decode_mode_kernel(const uint64_t* __restrict__ in, uint64_t nwords,
                        const unsigned long long* __restrict__ offsets, Geom g, General mode,
                        T* __restrict__ out) {
   typedef typename FT<T>::UInt UInt;
+  typedef ReadWords<D == 3 && HOW == kByTable> Words;
   constexpr int BS = 1 << (2 * D);
   extern __shared__ __align__(16) uint64_t smem[];
-  const Tables tables = stage_tables<D, T, true, kThreads>(smem);
-  tables_ready<D, T, true>();
-  SmemPlanes ps{smem + table_words<D, T, true>() + threadIdx.x, tables};
+  uint64_t* planes = smem;
+  Tables tables{nullptr, nullptr};
+  if constexpr (HOW == kByTable) {
+    tables = stage_tables<D, T, true, kThreads>(smem);
+    tables_ready<D, T, true>();
+    planes += table_words<D, T, true>();
+  }
+  SmemPlanes ps{planes + threadIdx.x, tables};
   const uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if (b >= g.nblocks) return;
   uint32_t ix, iy, iz;
   block_coords(g, b, ix, iy, iz);
-  BitReader<DevWords> r(DevWords{nullptr, in, nwords}, offsets[b]);
+  BitReader<Words> r(Words{in, nwords}, offsets[b]);
   UInt raw[BS];
-  decode_block_mode<D, T>(r, mode, raw, ps);
+  if constexpr (HOW == kByTable)
+    decode_block_mode<D, T>(r, mode, raw, ps);
+  else
+    decode_block_mode<D, T>(r, GeneralTokens<HOW == kByTokenTop32>(mode), raw, ps);
   scatter<D, T>(out, g, ix, iy, iz, raw);
 }
 
@@ -112,14 +126,34 @@ cudaError_t launch_encode_mode_t(const T* in, const Geom& g, const General& mode
   return cudaGetLastError();
 }
 
+// 4^3 blocks of integers go by token: their planes are dense from the first
+// ones on (300^3, precision 12, 20, 28: int32 by table 54, 68, 92 us, noisy 54,
+// 68, 118, by token 44, 57, 88, noisy 44, 57, 105).  So do those of floating
+// point with at most this many planes, too few to pay for the table (noisy and
+// smooth, by table / by token: floats, 16 planes 96, 74 / 93, 74, 18 planes 103,
+// 80 / 99, 84; doubles, 12 planes 136, 119 / 124, 113, 14 planes 152, 125, either
+// way).  The top 32 planes alone: int64, precision 12, 20, 28 79, 88, 102 -> 70,
+// 79, 93.
+template <typename T>
+constexpr uint32_t kTokenPrecision = sizeof(T) == 8 ? 12 : 16;
+
 template <int D, typename T>
 cudaError_t launch_decode_mode_t(const uint64_t* in, uint64_t nwords,
                                  const unsigned long long* offsets, const Geom& g,
                                  const General& mode, T* out, cudaStream_t s) {
   if (g.nblocks == 0) return cudaSuccess;
   const dim3 grid((unsigned)((g.nblocks + kThreads - 1) / kThreads));
-  const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0, table_words<D, T, true>());
-  auto k = decode_mode_kernel<D, T>;
+  auto k = decode_mode_kernel<D, T, D == 3 && FT<T>::INT ? kByToken : kByTable>;
+  bool tokens = D == 3 && FT<T>::INT;
+  if constexpr (D == 3) {
+    constexpr int kFew = FT<T>::P == 64 ? kByTokenTop32 : kByToken;
+    if (mode.maxprec <= (FT<T>::INT ? 32 : kTokenPrecision<T>)) {
+      k = decode_mode_kernel<D, T, kFew>;
+      tokens = true;
+    }
+  }
+  const size_t sm = smem_bytes(decode_slots<D, T>(), kStageNone, 0,
+                               tokens ? 0 : table_words<D, T, true>());
   cudaError_t e = allow_smem(k, sm);
   if (e != cudaSuccess) return e;
   k<<<grid, kThreads, sm, s>>>(in, nwords, offsets, g, mode, out);
