@@ -484,12 +484,11 @@ GZ_HD uint32_t rank_spread32(uint32_t z) {
 // most 16 bits and its whole code -- verbatim bits, then group tests -- at
 // most 16 + 33 bits, so it is built in 32-bit arithmetic and written in one
 // piece.  Same bits as the general form below.
-template <int BS, bool STOP_FULL = false, class W, class PlaneFn>
+template <int BS, class W, class PlaneFn>
 GZ_HD int code_planes_small(int k, int k_low, uint32_t& n, uint32_t& bits, W& w,
                             PlaneFn&& plane) {
   static_assert(BS <= 16, "at most 16 values per block");
-  // STOP_FULL: return as soon as every coefficient is significant
-  for (; k >= k_low && bits && !(STOP_FULL && n == (uint32_t)BS); k--) {
+  for (; k >= k_low && bits; k--) {
     const uint32_t x = (uint32_t)plane(k);
     const uint32_t bl = 32 - clz32(x);      // bit length of the plane
     const bool full = n == (uint32_t)BS;
@@ -616,11 +615,11 @@ GZ_HD bool group_in_window(uint64_t w, uint32_t bits, uint32_t& used, uint32_t& 
 // budget ends in included, goes through group_in_window, so a warp's lanes
 // do not split at their blocks' last planes (faster for 2D blocks of 32-bit
 // values; for 64-bit values and 4^3 blocks the split form measured faster).
-template <int BS, bool STOP_FULL = false, bool UNIFIED = false, class R, class StoreFn>
+template <int BS, bool UNIFIED = false, class R, class StoreFn>
 GZ_HD int uncode_planes_small(int k, int k_low, uint32_t& n, uint32_t& bits, R& r,
                               StoreFn&& store) {
   static_assert(BS <= 16, "at most 16 values per block");
-  for (; k >= k_low && bits && !(STOP_FULL && n == (uint32_t)BS); k--) {
+  for (; k >= k_low && bits; k--) {
     if constexpr (UNIFIED) {
       const uint32_t h = n < bits ? n : bits;  // verbatim bits (n == BS once all are significant)
       const uint64_t w = r.peek64();
@@ -691,7 +690,7 @@ GZ_HD int uncode_planes_small(int k, int k_low, uint32_t& n, uint32_t& bits, R& 
 template <int BS, bool UNIFIED = false, class R, class StoreFn>
 GZ_HD int uncode_planes(int k, int k_low, uint32_t& n, uint32_t& bits, R& r, StoreFn&& store) {
   if constexpr (BS <= 16)
-    return uncode_planes_small<BS, false, UNIFIED>(k, k_low, n, bits, r, store);
+    return uncode_planes_small<BS, UNIFIED>(k, k_low, n, bits, r, store);
   for (; k >= k_low && bits; k--) {
     const bool full = n == (uint32_t)BS;
     const uint32_t hlen = full ? (uint32_t)BS : n;
@@ -1074,7 +1073,7 @@ GZ_HD int uncode_runs01(UInt& u0, int k, int k_low, uint32_t& n, uint32_t& bits,
     // then, in the same step, one plane one at a time: one that brings a
     // new coefficient, the budget's last, or a plane past the window
     if (k < k_low || !bits) break;
-    k = uncode_planes_small<BS, false, UNIFIED>(k, k, n, bits, r, store);
+    k = uncode_planes_small<BS, UNIFIED>(k, k, n, bits, r, store);
   }
   return k;
 }

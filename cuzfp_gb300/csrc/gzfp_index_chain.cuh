@@ -36,8 +36,7 @@
 
 namespace gzfp {
 
-constexpr uint32_t kIndexMaxLen = 0x7fffu;   // longest block a table entry holds
-constexpr uint32_t kIndexNone = 0xffffffffu; // no exit, no entry
+constexpr uint32_t kIndexNone = 0xffffffffu;  // no exit, no entry
 
 struct IndexJob {
   const uint64_t* in;

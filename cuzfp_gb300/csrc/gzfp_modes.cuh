@@ -9,9 +9,8 @@
 // the lengths gives every block's start bit; every block's bits are then
 // moved to that position.  Decompression decodes every block from its start
 // bit when the offsets are known (the compressor returns them); otherwise
-// the starts are found first, by walkers over segments of the stream whose
-// chains are joined where they merge (below), or, failing that, by a single
-// thread walking every block in order.
+// the starts are found first, in parallel (gzfp_index_chain.cuh) or, of a few
+// dozen blocks, by one thread walking them in order (below).
 #pragma once
 
 #include "gzfp_kernels.cuh"
