@@ -220,10 +220,9 @@ __global__ void __launch_bounds__(kWalkThreads)
     index_walk_kernel(IndexJob j, IndexLists l, const IndexState* st) {
   typedef IndexStreamReader R;
   __shared__ IndexTables tables;
-  if (index_over(*st)) return;
+  const uint32_t n = index_over(*st) ? 0 : *l.count;
   stage_index_tables(&tables, kWalkThreads);
   __syncthreads();
-  const uint32_t n = *l.count;
   const R r{reinterpret_cast<const uint32_t*>(j.in), &tables, j.lo, j.nwords * 2};
   IndexLane<D, T, R> walk;
   bool live = false, more = true;

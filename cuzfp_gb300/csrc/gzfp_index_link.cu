@@ -34,8 +34,7 @@ __global__ void __launch_bounds__(kZeroThreads)
 __global__ void __launch_bounds__(kLinkThreads)
     index_exits_kernel(IndexJob j, const uint32_t* __restrict__ list,
                        const uint32_t* __restrict__ count, uint32_t* exits, const IndexState* st) {
-  if (index_over(*st)) return;
-  const uint32_t n = *count;
+  const uint32_t n = index_over(*st) ? 0 : *count;
   for (uint64_t i = (uint64_t)blockIdx.x * kLinkThreads + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * kLinkThreads) {
     const uint32_t p = list[i], s = p / j.seg_bits, w = p - s * j.seg_bits;

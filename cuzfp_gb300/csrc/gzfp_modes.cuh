@@ -131,10 +131,13 @@ cudaError_t launch_encode_mode_t(const T* in, const Geom& g, const General& mode
 // point with at most this many planes, too few to pay for the table (noisy and
 // smooth, by table / by token: floats, 16 planes 96, 74 / 93, 74, 18 planes 103,
 // 80 / 99, 84; doubles, 12 planes 136, 119 / 124, 113, 14 planes 152, 125, either
-// way).  The top 32 planes alone: int64, precision 12, 20, 28 79, 88, 102 -> 70,
-// 79, 93.
+// way), unless there are too few to give every scheduler a warp, where a block's
+// steps count, which are fewer by table (64 x 65 x 67 doubles, 12 planes 19 us,
+// by token 21; floats 11.5, 12.5).  The top 32 planes alone: int64, precision 12,
+// 20, 28 79, 88, 102 -> 70, 79, 93.
 template <typename T>
 constexpr uint32_t kTokenPrecision = sizeof(T) == 8 ? 12 : 16;
+constexpr uint64_t kTokenBlocks = 608 * 32;
 
 template <int D, typename T>
 cudaError_t launch_decode_mode_t(const uint64_t* in, uint64_t nwords,
@@ -146,7 +149,8 @@ cudaError_t launch_decode_mode_t(const uint64_t* in, uint64_t nwords,
   bool tokens = D == 3 && FT<T>::INT;
   if constexpr (D == 3) {
     constexpr int kFew = FT<T>::P == 64 ? kByTokenTop32 : kByToken;
-    if (mode.maxprec <= (FT<T>::INT ? 32 : kTokenPrecision<T>)) {
+    if (FT<T>::INT ? mode.maxprec <= 32
+                   : mode.maxprec <= kTokenPrecision<T> && g.nblocks > kTokenBlocks) {
       k = decode_mode_kernel<D, T, kFew>;
       tokens = true;
     }

@@ -36,6 +36,23 @@ def test_gpu_precisions(gz, orc, cuda, dt, kind):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dt", DTYPES)
+def test_gpu_many_blocks_of_few_planes(gz, orc, cuda, dt):
+    """Above and below the number of blocks from which few planes go by token."""
+    import torch
+    t = getattr(torch, np.dtype(dt).name)
+    for shape in ((108, 108, 107), (104, 108, 107)):
+        a = _field("smooth", shape, dt, 2)
+        for p in (3, 12, 13, 16, 17):
+            params = orc.mode_precision(dt, p)
+            s, offs = orc.compress_params(a, params, with_offsets=True)
+            w = torch.from_numpy(np.ascontiguousarray(s).view(np.int64)).to(cuda)
+            o = torch.from_numpy(offs.view(np.int64)).to(cuda)
+            y = gz.decompress_mode(w, shape, t, gz.Mode(*params), offsets=o)
+            assert _same(y, orc.decompress_params(s, shape, dt, params)), (shape, p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", DTYPES)
 def test_gpu_budgets(gz, orc, cuda, dt):
     import torch
     rng = np.random.default_rng(4)
