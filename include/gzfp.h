@@ -278,9 +278,12 @@ void gzfp_batch_default_config(gzfp_batch_config* cfg);
 const char* gzfp_batch_last_error(void);
 
 /* One batch, built and launched now (cfg may be NULL for the default).  The
-   library keeps one work list per device: a call first waits on the host
-   until the previous call's kernel, on whatever stream, has finished with
-   it, then queues its own work and returns. */
+   library keeps four work lists per device, each with three streams of its
+   own, and takes them in turn: a call waits on the host until the batch four
+   calls before it, on whatever stream, has finished with its list, then
+   queues its own work and returns, with up to three others still queued.
+   The grid kernels of a batch run side by side on `cuda_stream` and the
+   list's streams, joined before whatever follows on `cuda_stream`. */
 int gzfp_batch_compress(const gzfp_batch_item* items, int count, const gzfp_batch_config* cfg,
                         void* cuda_stream);
 int gzfp_batch_decompress(const gzfp_batch_item* items, int count, const gzfp_batch_config* cfg,
