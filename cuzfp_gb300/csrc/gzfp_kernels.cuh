@@ -224,9 +224,15 @@ struct BitReader<StagedWords<PITCH>> {
   uint32_t pos;  // bit position within the slot
   __device__ __forceinline__ BitReader(StagedWords<PITCH> w, uint64_t p)
       : buf(w.buf), pos((uint32_t)(p - (w.w0 << 6))) {}
+  // (window64 written out: called, the 512^3 double decoder takes 0.3% longer)
   __device__ __forceinline__ uint64_t peek64() const {
-    const uint32_t j = pos >> 6;
-    return window64(buf[j * PITCH], buf[(j + 1) * PITCH], pos & 63);
+    const uint32_t j = pos >> 6, s = pos & 63;
+    const uint64_t a = buf[j * PITCH], b = buf[(j + 1) * PITCH];
+    const uint32_t a0 = lo32(a), a1 = hi32(a), b0 = lo32(b), b1 = hi32(b);
+    const bool ge = s >= 32;
+    const uint32_t c0 = ge ? a1 : a0, c1 = ge ? b0 : a1, c2 = ge ? b1 : b0;
+    const uint32_t t = s & 31;
+    return ((uint64_t)__funnelshift_r(c1, c2, t) << 32) | __funnelshift_r(c0, c1, t);
   }
   __device__ __forceinline__ void skip(uint32_t n) { pos += n; }
   __device__ __forceinline__ uint64_t read(uint32_t n) {
